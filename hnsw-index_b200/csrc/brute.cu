@@ -3,12 +3,13 @@
 // kernels (src/kernels/x86.rs:32-131).
 //
 // Layout of the arithmetic: lane (c, l) = (lane >> 3, lane & 7) of a warp is
-// AVX2 accumulator chain c, vector lane l. A warp scores a micro-tile of
-// 4 queries x 8 rows: every lane runs the 32 FMA chains of its accumulator
-// for the 32 (query, row) pairs, then a butterfly transpose-reduce adds the
-// 32 accumulators of each pair in the reference order (bits 3, 4 of the lane
-// = chains (c0+c1),(c2+c3) then their sum; bit 2 = v_l + v_{l+4}; bit 0 then
-// bit 1 = the horizontal sum), leaving one pair's distance per lane.
+// AVX2 accumulator chain c, vector lane l, i.e. column `lane` of every 32. A
+// warp scores QW queries x RW rows (64 pairs): every lane runs the FMA chain
+// of its accumulator for each pair, two rows per packed f32x2 instruction;
+// then a transpose-reduce adds the 32 accumulators of each pair in the
+// reference order (lane bits 3, 4 = chains (c0+c1), (c2+c3), then their sum;
+// bit 2 = v_l + v_{l+4}; bit 0 then bit 1 = the horizontal sum), leaving two
+// rows' sums of one query in each lane.
 // Each block keeps a per-query top-k (by total_cmp distance, then key) of its
 // row slice; a merge kernel combines the slices.
 #include <algorithm>
@@ -16,43 +17,60 @@
 
 #include "common.cuh"
 #include "device.hpp"
+#include "warp_sort.cuh"
 
 namespace hnswgpu {
 namespace dev {
 
-constexpr int kQB = 16;      // queries per block (4 warps x 4)
-constexpr int kRT = 8;       // rows per tile
-
-// Orders (dk, row) entries by (distance key, key[row]).
-__device__ __forceinline__ bool entry_less(uint64_t a, uint64_t b, const uint64_t* __restrict__ keys) {
-    uint32_t da = uint32_t(a >> 32), db = uint32_t(b >> 32);
-    if (da != db) return da < db;
-    return __ldg(keys + uint32_t(a)) < __ldg(keys + uint32_t(b));
+// Top-k entries are (fkey(distance) << 32) | rank of the row's key, so the
+// u64 order is the reference's (total_cmp distance, key) order. The rank is
+// the row itself when the keys ascend (krank null).
+__device__ __forceinline__ uint64_t brute_entry(const BruteArgs& a, float dist, uint32_t row) {
+    return (uint64_t(fkey(dist)) << 32) | (a.krank ? __ldg(a.krank + row) : row);
 }
 
-// Warp-cooperative insert of x into the ascending list L[0, n) (room for one more).
-__device__ __forceinline__ void list_insert(uint64_t* L, uint32_t n, uint64_t x, const uint64_t* keys) {
-    const int lane = threadIdx.x & 31;
-    uint32_t pos = 0;
-    for (uint32_t b = 0; b < n; b += 32) {
-        uint32_t i = b + lane;
-        bool lt = i < n && entry_less(L[i], x, keys);
-        pos += __popc(__ballot_sync(kFull, lt));
-    }
-    if (n > pos)
-        for (int c = int((n - pos - 1) >> 5); c >= 0; --c) {
-            uint32_t i = pos + uint32_t(c) * 32 + lane;
-            bool mv = i < n;
-            uint64_t v = mv ? L[i] : 0;
-            __syncwarp();
-            if (mv) L[i + 1] = v;
-            __syncwarp();
-        }
-    if (lane == 0) L[pos] = x;
+// One query's top-k of a warp: an ascending list of n <= kk entries and a
+// buffer of cnt <= 32 entries still to be merged into it. Entries are
+// buffered so that one merge serves up to 32 of them.
+struct TopList {
+    uint64_t* L;
+    uint64_t* B;
+    uint32_t n, cnt;
+};
+
+__device__ __forceinline__ void top_flush(TopList& t, uint32_t kk) {
+    const int lane = lane_id();
+    const uint64_t x = uint32_t(lane) < t.cnt ? t.B[lane] : ~0ull;
+    const uint64_t worst = t.n == kk ? t.L[kk - 1] : ~0ull;
+    const uint32_t S = __ballot_sync(kFull, x < worst);
+    t.cnt = 0;
+    if (S == 0) return;
+    // The buffer is free once every lane holds its entry: it is the merge's scratch.
     __syncwarp();
+    batch_merge_gather(t.L, 0, t.n, S, x, kk, t.B);
+    __syncwarp();
+    t.n = min(t.n + uint32_t(__popc(S)), kk);
 }
 
-// vector::check + normalisation of each query (one warp per query).
+// Adds the entries x of the lanes in W (all lanes call); true if the buffer
+// was merged into the list for it.
+__device__ __forceinline__ bool top_push(TopList& t, uint32_t W, uint64_t x, uint32_t kk) {
+    const uint32_t c = __popc(W);
+    const bool full = t.cnt + c > 32;
+    if (full) top_flush(t, kk);
+    const int lane = lane_id();
+    if ((W >> lane) & 1u) t.B[t.cnt + __popc(W & ((1u << lane) - 1u))] = x;
+    t.cnt += c;
+    __syncwarp();
+    return full;
+}
+
+// vector::check + normalisation of each query (one warp per query). The f64
+// squared norm adds its terms in row order, as the reference does: the
+// products are formed 32 at a time, one per lane, and every lane adds them in
+// order (the chain of additions is all that is serial; one lane doing both
+// took 31 us for 768 dimensions). out_count and the lane minima start as "no
+// bound" for the score kernel.
 __global__ void brute_prep_kernel(BruteArgs a) {
     const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -60,23 +78,24 @@ __global__ void brute_prep_kernel(BruteArgs a) {
     const float* src = a.queries + size_t(q) * a.dim;
     float* dst = a.qprep + size_t(q) * a.dp;
     bool bad = false;
-    for (uint32_t i = lane; i < a.dp; i += 32) {
-        float x = i < a.dim ? src[i] : 0.0f;
+    double norm = 0.0;
+    for (uint32_t b = 0; b < a.dp; b += 32) {
+        const uint32_t i = b + uint32_t(lane);
+        const float x = i < a.dim ? src[i] : 0.0f;
         bad |= !isfinite(x);
         dst[i] = x;
+        const double p = __dmul_rn(double(x), double(x));
+        const uint32_t m = min(32u, a.dim - b);
+        if (m == 32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) norm = __dadd_rn(norm, __shfl_sync(kFull, p, j));
+        } else {
+            for (uint32_t j = 0; j < m; ++j) norm = __dadd_rn(norm, __shfl_sync(kFull, p, int(j)));
+        }
     }
     bad = __any_sync(kFull, bad);
-    __syncwarp();
     int32_t st = 0;
-    if (bad) st = 3;
-    double norm = 0.0;
-    if (!bad && lane == 0)
-        for (uint32_t i = 0; i < a.dim; ++i) {
-            double x = double(dst[i]);
-            norm = __dadd_rn(norm, __dmul_rn(x, x));
-        }
-    norm = __shfl_sync(kFull, norm, 0);
-    if (st == 0 && norm > double(3.40282346638528859812e+38F) / 8.0) st = 3;
+    if (bad || norm > double(3.40282346638528859812e+38F) / 8.0) st = 3;
     if (st == 0 && a.metric == 2) {
         if (norm == 0.0) st = 4;
         else {
@@ -84,31 +103,12 @@ __global__ void brute_prep_kernel(BruteArgs a) {
             for (uint32_t i = lane; i < a.dim; i += 32) dst[i] = __double2float_rn(__dmul_rn(double(dst[i]), inv));
         }
     }
-    if (lane == 0) a.out_status[q] = st;
-}
-
-// Butterfly transpose-reduce of 32 values per lane over the lane bits in
-// the order 3, 4, 2, 0, 1. Afterwards v[0] of lane L holds pair
-// p(L) = (b3 << 4) | (b4 << 3) | (b2 << 2) | (b0 << 1) | b1 of the bits of L.
-__device__ __forceinline__ float butterfly32(float (&v)[32], int lane) {
-    const int order[5] = {3, 4, 2, 0, 1};
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-        const int half = 16 >> s;
-        const bool hi = (lane >> order[s]) & 1;
-#pragma unroll
-        for (int j = 0; j < half; ++j) {
-            float send = hi ? v[j] : v[j + half];
-            float keep = hi ? v[j + half] : v[j];
-            float recv = __shfl_xor_sync(kFull, send, 1 << order[s]);
-            v[j] = __fadd_rn(keep, recv);
-        }
+    if (lane == 0) {
+        a.out_status[q] = st;
+        a.out_count[q] = 0xFFFFFFFFu;
     }
-    return v[0];
-}
-
-__device__ __forceinline__ int pair_of_lane(int L) {
-    return (((L >> 3) & 1) << 4) | (((L >> 4) & 1) << 3) | (((L >> 2) & 1) << 2) | ((L & 1) << 1) | ((L >> 1) & 1);
+    if (a.minima)
+        for (uint32_t i = lane; i < kBruteMinima; i += 32) a.minima[size_t(q) * kBruteMinima + i] = 0xFFFFFFFFu;
 }
 
 // Whether query q admits row r under the optional filter.
@@ -120,170 +120,449 @@ __device__ __forceinline__ bool brute_admits(const BruteArgs& a, uint32_t q, uin
     return bit < a.filter_nbits && ((__ldg(bits + (bit >> 6)) >> (bit & 63)) & 1ull);
 }
 
+// Two f32 operations per instruction, each rounded as its scalar form.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// acc += (q + r)^2 (L2: q is staged negated, and (r - q)^2 is (q - r)^2 bit
+// for bit) or q * r, element by element.
 template <bool L2>
-__global__ void __launch_bounds__(128) brute_score_kernel(BruteArgs a, uint32_t kk) {
-    extern __shared__ __align__(16) char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t dp = a.dp;
-    float* sq = reinterpret_cast<float*>(smem);                 // kQB * dp
-    float* sr = sq + size_t(kQB) * dp;                           // kRT * dp
-    uint64_t* lists = reinterpret_cast<uint64_t*>(sr + size_t(kRT) * dp);  // kQB * (kk + 1)
-    const uint32_t q0 = blockIdx.x * kQB;
-    const uint32_t slice = blockIdx.y, nslices = gridDim.y;
-    const uint32_t rows_per = (a.n + nslices - 1) / nslices;
-    const uint32_t r_begin = min(a.n, slice * rows_per), r_end = min(a.n, r_begin + rows_per);
-    // Stage the block's prepared queries.
-    for (uint32_t i = threadIdx.x; i < kQB * dp; i += blockDim.x) {
-        uint32_t qq = i / dp, j = i % dp;
-        sq[i] = (q0 + qq < a.nq) ? a.qprep[size_t(q0 + qq) * dp + j] : 0.0f;
-    }
-    // Per-query list sizes live in registers of the owning warp.
-    uint32_t lsize[4] = {0, 0, 0, 0};
-    __syncthreads();
-    const uint32_t nfull = a.dim >> 5;
-    const uint32_t rem8 = (a.dim & 31) >> 3;
-    const uint32_t tail0 = (nfull << 5) + (rem8 << 3);
-    const int p = pair_of_lane(lane);
-    const int my_q = p >> 3, my_r = p & 7;  // pair p = 8 * query + row
-    for (uint32_t t0 = r_begin; t0 < r_end; t0 += kRT) {
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kRT * dp / 4; i += blockDim.x) {
-            uint32_t rr = (i * 4) / dp, j = (i * 4) % dp;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t0 + rr < r_end) v = ldg_f4(a.base + size_t(t0 + rr) * dp + j);
-            *reinterpret_cast<float4*>(sr + rr * dp + j) = v;
-        }
-        __syncthreads();
-        float acc[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
-        const float* qw = sq + size_t(warp * 4) * dp;
-        for (uint32_t k = 0; k < nfull; ++k) {
-            float qv[4], rv[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) qv[i] = qw[size_t(i) * dp + 32 * k + lane];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) rv[i] = sr[size_t(i) * dp + 32 * k + lane];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (L2) {
-                        float d = __fsub_rn(qv[i], rv[j]);
-                        acc[8 * i + j] = __fmaf_rn(d, d, acc[8 * i + j]);
-                    } else {
-                        acc[8 * i + j] = __fmaf_rn(qv[i], rv[j], acc[8 * i + j]);
-                    }
-                }
-        }
-        // 8-wide remainder blocks into chain 0 (lanes 0..7).
-        if (lane < 8)
-            for (uint32_t s = 0; s < rem8; ++s) {
-                const uint32_t e = 32 * nfull + 8 * s + lane;
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float x = qw[size_t(i) * dp + e], y = sr[size_t(j) * dp + e];
-                        if (L2) {
-                            float d = __fsub_rn(x, y);
-                            acc[8 * i + j] = __fmaf_rn(d, d, acc[8 * i + j]);
-                        } else {
-                            acc[8 * i + j] = __fmaf_rn(x, y, acc[8 * i + j]);
-                        }
-                    }
-            }
-        float s = butterfly32(acc, lane);
-        for (uint32_t e = tail0; e < a.dim; ++e) {
-            float x = qw[size_t(my_q) * dp + e], y = sr[size_t(my_r) * dp + e];
-            if (L2) {
-                float d = __fsub_rn(x, y);
-                s = __fadd_rn(s, __fmul_rn(d, d));
-            } else {
-                s = __fadd_rn(s, __fmul_rn(x, y));
-            }
-        }
-        const float dist = metric_from_sum(a.metric, s);
-        const uint32_t row = t0 + uint32_t(my_r);
-        const uint32_t qg = q0 + uint32_t(warp * 4 + my_q);
-        const bool valid = row < r_end && qg < a.nq && brute_admits(a, qg, row);
-        const uint64_t cand = (uint64_t(fkey(dist)) << 32) | row;
-        // Per-query top-k update (rare after warm-up).
-#pragma unroll
-        for (int qq = 0; qq < 4; ++qq) {
-            uint64_t* L = lists + size_t(warp * 4 + qq) * (kk + 1);
-            const uint32_t n = lsize[qq];
-            bool want = valid && my_q == qq && (n < kk || entry_less(cand, L[n - 1], a.keys));
-            uint32_t W = __ballot_sync(kFull, want);
-            while (W) {
-                const int src = __ffs(W) - 1;
-                W &= W - 1;
-                const uint64_t x = __shfl_sync(kFull, cand, src);
-                uint32_t m = lsize[qq];
-                if (m >= kk && !entry_less(x, L[m - 1], a.keys)) continue;
-                list_insert(L, m, x, a.keys);
-                lsize[qq] = min(m + 1, kk);
-            }
-        }
-    }
-    // Write this slice's partial lists.
-    for (int qq = 0; qq < 4; ++qq) {
-        const uint32_t qg = q0 + uint32_t(warp * 4 + qq);
-        if (qg >= a.nq) continue;
-        const uint64_t* L = lists + size_t(warp * 4 + qq) * (kk + 1);
-        uint64_t* out = a.part + (size_t(qg) * nslices + slice) * kk;
-        for (uint32_t i = lane; i < kk; i += 32) out[i] = i < lsize[qq] ? L[i] : ~0ull;
+__device__ __forceinline__ void acc_pair(uint64_t& acc, uint64_t q, uint64_t r) {
+    if (L2) {
+        const uint64_t d = add2(q, r);
+        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc) : "l"(d));
+    } else {
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(q), "l"(r));
     }
 }
 
-// Merges the per-slice lists of each query (one warp per query): repeated
-// minimum over the slice heads, ties broken by key.
-__global__ void brute_merge_kernel(BruteArgs a, uint32_t kk, uint32_t nslices) {
-    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (q >= a.nq) return;
-    if (a.out_status[q] != 0 || a.k == 0) {
-        if (lane == 0) a.out_count[q] = 0;
-        return;
-    }
-    const uint64_t* P = a.part + size_t(q) * nslices * kk;
-    uint32_t head[2] = {0, 0};  // lanes own slices lane and lane + 32
-    const uint32_t want = min(a.k, a.n);
-    uint32_t got = 0;
-    for (; got < want; ++got) {
-        uint64_t best = ~0ull;
-        int bs = -1;
+// One stage of the transpose-reduce: of the first N accumulators a lane keeps
+// half and adds the partner lane's values of the same pairs. With PERM the
+// lane's accumulators are laid out so that it always keeps the lower half
+// (the queries were read in an order that depends on the lane); otherwise its
+// lane bit selects the half.
+template <int N, bool PERM, int ALL>
+__device__ __forceinline__ void fold_pairs(uint64_t (&v)[ALL], int bit, bool hi) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t s = uint32_t(lane) + 32u * h;
-            if (s < nslices && head[h] < kk) {
-                uint64_t v = P[size_t(s) * kk + head[h]];
-                if (v != ~0ull && (bs < 0 || entry_less(v, best, a.keys))) {
-                    best = v;
-                    bs = int(s);
+    for (int p = 0; p < N / 2; ++p) {
+        const uint64_t send = !PERM && hi ? v[p] : v[p + N / 2];
+        const uint64_t keep = !PERM && hi ? v[p + N / 2] : v[p];
+        v[p] = add2(keep, __shfl_xor_sync(kFull, send, bit));
+    }
+}
+
+// Shape of the score kernel: WQ x WR warps, each scoring QW queries x RW rows
+// (64 pairs) of the block's tile of QB queries x RB rows. Rows stream through
+// a ring of kStages chunks of KC columns filled by cp.async; the queries stay
+// in shared memory, chunk by chunk. Row strides are padded by four floats so
+// that a column of rows spreads over the banks (the scalar tail reads one;
+// the queries' tails have a padded array of their own).
+template <int QW_, int RW_, int WQ_, int WR_>
+struct BruteTile {
+    static constexpr int QW = QW_, RW = RW_, WQ = WQ_, WR = WR_;
+    static constexpr int QB = QW * WQ, RB = RW * WR, kWarps = WQ * WR, kThreads = 32 * kWarps;
+    // With one warp along the queries a row belongs to one warp, which then
+    // copies its own rows and waits for nobody else.
+    static constexpr bool kPrivate = WQ == 1;
+    static constexpr int KC = RB >= 128 ? 32 : (RB >= 32 ? 64 : 128);
+    static constexpr int kStages = kPrivate ? 4 : 3;
+    static constexpr int kRowStride = KC + 4;
+    static constexpr size_t kRingBytes = size_t(kStages) * RB * kRowStride * 4;
+    static constexpr size_t kBufBytes = size_t(kWarps) * QW * 32 * 8;
+    static constexpr int kTailStride = 9;  // tail columns (at most 7) of a query
+    static size_t smem(uint32_t dp, uint32_t list_kk) {
+        return size_t((dp + KC - 1) / KC) * QB * KC * 4 + size_t(QB) * kTailStride * 4 + kRingBytes + kBufBytes +
+               size_t(kWarps) * QW * (size_t(list_kk) * 8 + 8);
+    }
+};
+
+// Lists longer than this live in the partial-result array instead of shared
+// memory (a list is only touched by a merge of up to 32 entries).
+constexpr uint32_t kSharedListMax = 128;
+
+// Smallest x (to 1/4096 of the range below hi) such that at least k of the
+// values v (M per lane, of four neighboring lanes together) are <= x; hi when
+// there are fewer.
+template <int M>
+__device__ __forceinline__ uint32_t kth_bound(const uint32_t (&v)[M], uint32_t k, uint32_t hi) {
+    hi = min(hi, __shfl_xor_sync(kFull, hi, 1));
+    hi = min(hi, __shfl_xor_sync(kFull, hi, 2));
+    uint32_t lo = hi;
+#pragma unroll
+    for (int i = 0; i < M; ++i) lo = min(lo, v[i]);
+    lo = min(lo, __shfl_xor_sync(kFull, lo, 1));
+    lo = min(lo, __shfl_xor_sync(kFull, lo, 2));
+    // `hi` is a bound (or the one given), below `lo` there are fewer than k.
+#pragma unroll 1
+    for (int it = 0; it < 12; ++it) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        uint32_t c = 0;
+#pragma unroll
+        for (int i = 0; i < M; ++i) c += v[i] <= mid ? 1u : 0u;
+        c += __shfl_xor_sync(kFull, c, 1);
+        c += __shfl_xor_sync(kFull, c, 2);
+        if (c >= k) hi = mid;
+        else lo = mid;
+    }
+    return hi;
+}
+
+// Scores every row of a slice against the block's queries and keeps each
+// query's best kk. An entry costs about as much to insert as a tile of pairs
+// to score, so the lists share bounds per query; a distance above one cannot
+// be among the best kk. One bound is the smallest kk-th distance of any list
+// (out_count, atomicMin). The other, which works long before the lists are
+// full, comes from the minima of the lanes: the lanes that finish a query's
+// pairs see disjoint rows, so the kk-th smallest of their minima bounds the
+// kk-th distance of all. They are published and read after 1, 3, 7, ... tiles
+// (a reader may see some of them late: every value is a real row's distance).
+template <bool L2, class T>
+__global__ void __launch_bounds__(T::kThreads, T::kThreads == 128 ? 4 : 8) brute_score_kernel(BruteArgs a, uint32_t kk,
+                                                                                            uint32_t rows_per,
+                                                                                            uint32_t nslices) {
+    constexpr int QW = T::QW, RW = T::RW, RP = RW / 2, NP = QW * RP;
+    static_assert(NP == 32, "a lane ends with one packed pair of rows of one query");
+    static_assert((T::QB * T::kTailStride) % 2 == 0, "8-byte alignment of the lists");
+    extern __shared__ __align__(16) char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wq = warp % T::WQ, wr = warp / T::WQ;
+    const uint32_t dp = a.dp;
+    const uint32_t nk = (dp + T::KC - 1) / T::KC;
+    const bool shared_lists = kk <= kSharedListMax;
+    float* sq = reinterpret_cast<float*>(smem);
+    float* sr = sq + size_t(nk) * T::QB * T::KC;
+    float* sqt = sr + T::kRingBytes / 4;
+    uint64_t* bufs = reinterpret_cast<uint64_t*>(sqt + T::QB * T::kTailStride);
+    uint2* meta = reinterpret_cast<uint2*>(reinterpret_cast<char*>(bufs) + T::kBufBytes);  // per list: (n, cnt)
+    uint64_t* lists = reinterpret_cast<uint64_t*>(meta + T::kWarps * QW);
+    const uint32_t q0 = blockIdx.x * T::QB, slice = blockIdx.y;
+    const uint32_t r_begin = min(a.n, slice * rows_per), r_end = min(a.n, r_begin + rows_per);
+    const uint32_t wq0 = q0 + uint32_t(wq * QW);  // this warp's first query
+    const bool active = wq0 < a.nq;
+    uint64_t* wbuf = bufs + size_t(warp) * QW * 32;
+    uint2* wmeta = meta + warp * QW;
+    // The list of warp w's query i: shared memory, or (one warp per query
+    // then, T::WR == 1) the slice's list in the partial-result array.
+    auto list_of = [&](int w, int i) -> uint64_t* {
+        if (shared_lists) return lists + (size_t(w) * QW + i) * kk;
+        const uint32_t q = min(q0 + uint32_t((w % T::WQ) * QW + i), a.nq - 1);
+        return a.part + (size_t(q) * nslices + slice) * kk;
+    };
+    for (uint32_t i = threadIdx.x; i < T::QB * (dp >> 2); i += T::kThreads) {
+        const uint32_t qq = i / (dp >> 2), j = (i % (dp >> 2)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (q0 + qq < a.nq) v = *reinterpret_cast<const float4*>(a.qprep + size_t(q0 + qq) * dp + j);
+        if (L2) v = make_float4(-v.x, -v.y, -v.z, -v.w);
+        *reinterpret_cast<float4*>(sq + (j / T::KC * T::QB + qq) * T::KC + j % T::KC) = v;
+    }
+    if (lane < QW) wmeta[lane] = make_uint2(0, 0);
+    const uint32_t nfull = a.dim >> 5, rem8 = (a.dim & 31) >> 3, tail0 = (nfull << 5) + (rem8 << 3);
+    const uint32_t ntail = a.dim - tail0;
+    for (uint32_t i = threadIdx.x; i < T::QB * 8; i += T::kThreads) {
+        const uint32_t qq = i >> 3, e = i & 7;
+        if (e < ntail && q0 + qq < a.nq) {
+            const float v = a.qprep[size_t(q0 + qq) * dp + tail0 + e];
+            sqt[qq * T::kTailStride + e] = L2 ? -v : v;
+        }
+    }
+    const uint32_t ntiles = (r_end - r_begin + T::RB - 1) / T::RB, total = ntiles * nk;
+    // Copies the next chunk (kc_next of the row tile at row_next) into stage
+    // s_next; rows past the slice repeat its last.
+    constexpr uint32_t P = T::KC / 4;
+    const uint32_t who = T::kPrivate ? uint32_t(lane) : threadIdx.x;
+    const uint32_t my_c = (who % P) * 4, my_r = (T::kPrivate ? uint32_t(wr * RW) : 0u) + who / P;
+    uint32_t issued = 0, kc_next = 0, row_next = r_begin + my_r, s_next = 0;
+    auto advance = [&]() {
+        if (issued < total) {
+            const uint32_t col = kc_next * T::KC + my_c;
+            if (col < dp) {
+                float* dst = sr + (s_next * T::RB + my_r) * T::kRowStride + my_c;
+#pragma unroll
+                for (uint32_t r = 0; r < uint32_t(T::kPrivate ? RW : T::RB);
+                     r += (T::kPrivate ? 32 : T::kThreads) / P) {
+                    const uint32_t row = min(row_next + r, r_end - 1);
+                    cp_async16(dst + r * T::kRowStride, a.base + size_t(row) * dp + col);
+                }
+            }
+            if (++kc_next == nk) {
+                kc_next = 0;
+                row_next += T::RB;
+            }
+            s_next = s_next + 1 == T::kStages ? 0 : s_next + 1;
+            ++issued;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int s = 0; s < T::kStages - 1; ++s) advance();
+    __syncthreads();
+    // The pairs this lane finishes: rows 2 my_p, 2 my_p + 1 of query my_q.
+    const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
+    const int p0 = (b3 ? 16 : 0) + (b4 ? 8 : 0) + (b2 ? 4 : 0) + (b0 ? 2 : 0) + (b1 ? 1 : 0);
+    const int my_q = p0 / RP, my_p = p0 % RP;
+    uint32_t thr = 0xFFFFFFFFu;   // bound of my_q
+    uint32_t best = 0xFFFFFFFFu;  // smallest admitted distance this lane finished
+    const uint32_t mslot = (slice * T::WR + uint32_t(wr)) * RP + uint32_t(my_p);
+    const uint32_t nmin = min(nslices * T::WR * RP, kBruteMinima);
+    const bool use_minima = a.minima != nullptr && nmin >= kk;
+    const uint32_t q = wq0 + uint32_t(my_q);
+    const float* qw = sq + wq * QW * T::KC + lane;
+    uint32_t stage = 0;
+    for (uint32_t tile = 0; tile < ntiles; ++tile) {
+        uint64_t acc[NP];  // query i ^ my_q, rows 2j and 2j + 1 at i * RP + j
+#pragma unroll
+        for (int p = 0; p < NP; ++p) acc[p] = 0ull;
+        const float* rw = nullptr;
+        for (uint32_t kc = 0; kc < nk; ++kc) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(T::kStages - 2) : "memory");
+            if (T::kPrivate) __syncwarp();
+            else __syncthreads();
+            advance();
+            rw = sr + (stage * T::RB + wr * RW) * T::kRowStride;
+            stage = stage + 1 == T::kStages ? 0 : stage + 1;
+            if (!active) continue;
+            const float* rk = rw + lane;
+            const float* qk = qw + kc * (T::QB * T::KC);
+            const float* qp[QW];
+#pragma unroll
+            for (int i = 0; i < QW; ++i) qp[i] = qk + (i ^ my_q) * T::KC;
+            auto step = [&](uint32_t col) {
+                uint64_t rv[RP];
+#pragma unroll
+                for (int j = 0; j < RP; ++j)
+                    rv[j] = pack2(rk[2 * j * T::kRowStride + col], rk[(2 * j + 1) * T::kRowStride + col]);
+#pragma unroll
+                for (int i = 0; i < QW; ++i) {
+                    const float x = qp[i][col];
+                    const uint64_t xx = pack2(x, x);
+#pragma unroll
+                    for (int j = 0; j < RP; ++j) acc_pair<L2>(acc[i * RP + j], xx, rv[j]);
+                }
+            };
+            // Full steps of the chunk, then (last chunk) the 8-wide remainder
+            // blocks, which go into chain 0 (lanes 0..7).
+            const uint32_t k0 = kc * (T::KC / 32), full = 32 * min(uint32_t(T::KC / 32), nfull - min(nfull, k0));
+            if (full == T::KC) {
+#pragma unroll
+                for (uint32_t col = 0; col < T::KC; col += 32) step(col);
+            } else {
+#pragma unroll 1
+                for (uint32_t col = 0; col < full; col += 32) step(col);
+                if (lane < 8)
+#pragma unroll 1
+                    for (uint32_t s = 0; s < rem8; ++s) step(full + 8 * s);
+                __syncwarp();
+            }
+        }
+        if (!active) continue;
+        const uint32_t shared_thr = q < a.nq ? __ldcg(a.out_count + q) : 0u;
+        fold_pairs<32, true>(acc, 8, b3);
+        fold_pairs<16, QW == 8>(acc, 16, b4);
+        fold_pairs<8, QW == 8>(acc, 4, b2);
+        fold_pairs<4, false>(acc, 1, b0);
+        fold_pairs<2, false>(acc, 2, b1);
+        if (use_minima && tile > 0 && (tile & (tile + 1)) == 0) {
+            // Published one tile ago (tile + 1 a power of two).
+            constexpr int M = kBruteMinima / 4;
+            uint32_t m[M];
+            const uint4* src = reinterpret_cast<const uint4*>(a.minima + size_t(min(q, a.nq - 1)) * kBruteMinima);
+#pragma unroll
+            for (int i = 0; i < M / 4; ++i) {
+                const uint4 t4 = __ldcg(src + (lane & 3) * (M / 4) + i);
+                m[4 * i] = t4.x;
+                m[4 * i + 1] = t4.y;
+                m[4 * i + 2] = t4.z;
+                m[4 * i + 3] = t4.w;
+            }
+            thr = min(thr, kth_bound(m, kk, thr));
+        }
+        const float2 sums = unpack2(acc[0]);
+        float s[2] = {sums.x, sums.y};
+        const float* rt = rw + 2 * my_p * T::kRowStride + tail0 - (nk - 1) * T::KC;
+        const float* qt = sqt + (wq * QW + my_q) * T::kTailStride;
+        for (uint32_t e = 0; e < ntail; ++e) {
+            const float x = qt[e];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const float y = rt[v * T::kRowStride + e];
+                if (L2) {
+                    const float d = __fadd_rn(x, y);
+                    s[v] = __fadd_rn(s[v], __fmul_rn(d, d));
+                } else {
+                    s[v] = __fadd_rn(s[v], __fmul_rn(x, y));
                 }
             }
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            uint64_t ob = __shfl_xor_sync(kFull, best, off);
-            int os = __shfl_xor_sync(kFull, bs, off);
-            bool take = os >= 0 && (bs < 0 || entry_less(ob, best, a.keys) ||
-                                    (!entry_less(best, ob, a.keys) && os < bs));
-            if (take) {
-                best = ob;
-                bs = os;
+        const uint32_t row0 = r_begin + tile * T::RB + uint32_t(wr * RW + 2 * my_p);
+        const uint32_t dk0 = fkey(metric_from_sum(a.metric, s[0])), dk1 = fkey(metric_from_sum(a.metric, s[1]));
+        thr = min(thr, shared_thr);
+        bool want0 = dk0 <= thr && row0 < r_end && q < a.nq;
+        bool want1 = dk1 <= thr && row0 + 1 < r_end && q < a.nq;
+        if (a.filter_bits) {
+            want0 = want0 && brute_admits(a, q, row0);
+            want1 = want1 && brute_admits(a, q, row0 + 1);
+        }
+        if (want0) best = min(best, dk0);
+        if (want1) best = min(best, dk1);
+        if (use_minima && ((tile + 1) & (tile + 2)) == 0 && mslot < kBruteMinima && q < a.nq)
+            __stcg(a.minima + size_t(q) * kBruteMinima + mslot, best);
+        if (!__any_sync(kFull, want0 || want1)) continue;
+#pragma unroll 1
+        for (uint32_t v = 0; v < 2; ++v) {
+            const bool want = v ? want1 : want0;
+            const uint32_t row = row0 + v;
+            uint64_t e = (uint64_t(v ? dk1 : dk0) << 32) | row;
+            if (want && a.krank) e = (e & 0xFFFFFFFF00000000ull) | __ldg(a.krank + row);
+            uint32_t W = __ballot_sync(kFull, want);
+            while (W) {
+                // The lanes of one query at a time.
+                const int src = __ffs(int(W)) - 1;
+                const int qi = __shfl_sync(kFull, my_q, src);
+                const uint32_t Wi = W & __ballot_sync(kFull, my_q == qi);
+                W &= ~Wi;
+                TopList t{list_of(warp, qi), wbuf + qi * 32, wmeta[qi].x, wmeta[qi].y};
+                const bool merged = top_push(t, Wi, e, kk);
+                if (lane == 0) wmeta[qi] = make_uint2(t.n, t.cnt);
+                __syncwarp();
+                // A merge happened: the list's last entry is a new bound.
+                if (merged && t.n == kk) {
+                    const uint32_t last = uint32_t(t.L[kk - 1] >> 32);
+                    if (my_q == qi) thr = min(thr, last);
+                    if (lane == 0) atomicMin(a.out_count + wq0 + qi, last);
+                }
             }
         }
-        if (bs < 0) break;
-        if (uint32_t(bs) == uint32_t(lane)) head[0]++;
-        if (uint32_t(bs) == uint32_t(lane) + 32) head[1]++;
-        if (lane == 0) {
-            a.out_keys[size_t(q) * a.k + got] = __ldg(a.keys + uint32_t(best));
-            a.out_dist[size_t(q) * a.k + got] = kdec(uint32_t(best >> 32));
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (active) {
+        for (int i = 0; i < QW; ++i) {
+            TopList t{list_of(warp, i), wbuf + i * 32, wmeta[i].x, wmeta[i].y};
+            __syncwarp();
+            if (t.cnt) top_flush(t, kk);
+            if (lane == 0) wmeta[i] = make_uint2(t.n, 0);
+            __syncwarp();
         }
     }
-    if (lane == 0) a.out_count[q] = got;
+    __syncthreads();
+    // The lists of the WR warps that share queries become one, written out by
+    // the first of them (unused entries ~0).
+    if (!active || wr != 0) return;
+    for (int i = 0; i < QW; ++i) {
+        const uint32_t qg = wq0 + uint32_t(i);
+        if (qg >= a.nq) break;
+        TopList t{list_of(warp, i), wbuf + i * 32, wmeta[i].x, 0};
+        for (int r = 1; r < T::WR; ++r) {
+            const int w2 = wq + r * T::WQ;
+            const uint64_t* other = list_of(w2, i);
+            const uint32_t n2 = meta[w2 * QW + i].x;
+            for (uint32_t b = 0; b < n2; b += 32) {
+                const uint64_t x = b + uint32_t(lane) < n2 ? other[b + lane] : ~0ull;
+                const uint64_t worst = t.n == kk ? t.L[kk - 1] : ~0ull;
+                const uint32_t S = __ballot_sync(kFull, x < worst);
+                if (S == 0) break;
+                batch_merge_gather(t.L, 0, t.n, S, x, kk, t.B);
+                __syncwarp();
+                t.n = min(t.n + uint32_t(__popc(S)), kk);
+            }
+        }
+        uint64_t* out = a.part + (size_t(qg) * nslices + slice) * kk;
+        if (shared_lists) {
+            for (uint32_t j = lane; j < kk; j += 32) out[j] = j < t.n ? t.L[j] : ~0ull;
+        } else {
+            for (uint32_t j = t.n + lane; j < kk; j += 32) out[j] = ~0ull;
+        }
+    }
+}
+
+// Merges the per-slice lists of each query: a block per query, each warp
+// taking a share of the entries, filtered by the query's shared bound, into
+// a list of its own; warp 0 merges those and writes the results.
+constexpr uint32_t kHeads = 4;  // list heads per thread
+__global__ void brute_merge_kernel(BruteArgs a, uint32_t kk, uint32_t nslices) {
+    extern __shared__ __align__(16) char smem[];
+    const uint32_t q = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (a.out_status[q] != 0 || a.k == 0 || a.n == 0) {
+        if (threadIdx.x == 0) a.out_count[q] = 0;
+        return;
+    }
+    uint64_t* lists = reinterpret_cast<uint64_t*>(smem);
+    uint64_t* bufs = lists + size_t(nw) * kk;
+    uint32_t* sizes = reinterpret_cast<uint32_t*>(bufs + size_t(nw) * 32);
+    const uint64_t* P = a.part + size_t(q) * nslices * kk;
+    const uint64_t n = uint64_t(nslices) * kk;
+    // Entries above `bound` cannot be results: the score kernel's shared bound
+    // and the kk-th smallest list head.
+    uint32_t bound = a.out_count[q];
+    if (nslices >= kk && nslices <= blockDim.x * kHeads) {
+        uint32_t h[kHeads];
+#pragma unroll
+        for (uint32_t j = 0; j < kHeads; ++j) {
+            const uint32_t s = threadIdx.x + j * blockDim.x;
+            h[j] = s < nslices ? uint32_t(__ldcg(P + size_t(s) * kk) >> 32) : 0xFFFFFFFFu;
+        }
+        uint32_t lo = 0, hi = bound;
+        for (int it = 0; it < 24 && hi - lo > 1; ++it) {
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < kHeads; ++j)
+                if (j * blockDim.x < nslices) c += uint32_t(__syncthreads_count(h[j] <= mid));
+            if (c >= kk) hi = mid;
+            else lo = mid;
+        }
+        bound = hi;
+    }
+    TopList t{lists + size_t(warp) * kk, bufs + warp * 32, 0, 0};
+    uint64_t worst = bound == 0xFFFFFFFFu ? ~0ull : (uint64_t(bound) + 1) << 32;  // entries below may be results
+    for (uint64_t b0 = uint64_t(warp) * 128; b0 < n; b0 += uint64_t(nw) * 128) {
+        uint64_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t i = b0 + uint64_t(32 * j + lane);
+            v[j] = i < n ? P[i] : ~0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t W = __ballot_sync(kFull, v[j] < worst);
+            if (W == 0) continue;
+            top_push(t, W, v[j], kk);
+            if (t.n == kk) worst = min(worst, t.L[kk - 1]);
+        }
+    }
+    if (t.cnt) top_flush(t, kk);
+    if (lane == 0) sizes[warp] = t.n;
+    __syncthreads();  // every thread has read the bound that out_count held
+    if (warp != 0) return;
+    for (int w2 = 1; w2 < nw; ++w2) {
+        const uint64_t* L2p = lists + size_t(w2) * kk;
+        const uint32_t n2 = sizes[w2];
+        for (uint32_t b = 0; b < n2; b += 32) {
+            const uint64_t x = b + uint32_t(lane) < n2 ? L2p[b + lane] : ~0ull;
+            const uint32_t S = __ballot_sync(kFull, x < (t.n == kk ? t.L[kk - 1] : ~0ull));
+            if (S == 0) break;
+            batch_merge_gather(t.L, 0, t.n, S, x, kk, t.B);
+            __syncwarp();
+            t.n = min(t.n + uint32_t(__popc(S)), kk);
+        }
+    }
+    const uint32_t want = min(t.n, min(a.k, a.n));
+    for (uint32_t i = lane; i < want; i += 32) {
+        a.out_keys[size_t(q) * a.k + i] = __ldg(a.skeys + uint32_t(t.L[i]));
+        a.out_dist[size_t(q) * a.k + i] = kdec(uint32_t(t.L[i] >> 32));
+    }
+    if (lane == 0) a.out_count[q] = want;
 }
 
 // Exact re-rank of tensor-core candidates (one warp per query): every
@@ -297,9 +576,10 @@ __global__ void brute_rerank_kernel(BruteArgs a, const uint64_t* __restrict__ ca
     extern __shared__ __align__(16) char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t q = blockIdx.x * (blockDim.x >> 5) + uint32_t(warp);
-    uint64_t* L = reinterpret_cast<uint64_t*>(smem) + size_t(warp) * (kk + 1);
-    uint32_t* pos = reinterpret_cast<uint32_t*>(reinterpret_cast<uint64_t*>(smem) + size_t(blockDim.x >> 5) * (kk + 1)) +
-                    warp * 32;
+    const uint32_t nw = blockDim.x >> 5;
+    uint64_t* lists = reinterpret_cast<uint64_t*>(smem);
+    uint64_t* bufs = lists + size_t(nw) * kk;
+    uint32_t* pos = reinterpret_cast<uint32_t*>(bufs + size_t(nw) * 32) + warp * 32;
     if (q >= a.nq) return;
     if (a.out_status[q] != 0) {
         if (lane == 0) a.out_count[q] = 0;
@@ -314,7 +594,7 @@ __global__ void brute_rerank_kernel(BruteArgs a, const uint64_t* __restrict__ ca
     const float* qv = a.qprep + size_t(q) * a.dp;
     const uint64_t* C = cand + size_t(q) * cand_cap;
     const int g = lane >> 3, g8 = lane & 7;
-    uint32_t size = 0;
+    TopList t{lists + size_t(warp) * kk, bufs + warp * 32, 0, 0};
     for (uint32_t base = 0; base < total; base += 32) {
         const uint32_t i = base + uint32_t(lane);
         uint32_t row = 0;
@@ -334,24 +614,20 @@ __global__ void brute_rerank_kernel(BruteArgs a, const uint64_t* __restrict__ ca
             const float* xr = a.base + size_t(rrow) * a.dp;
             float sum = a.metric == 0 ? group_sum<true>(xr, qv, int(a.dim), g8) : group_sum<false>(xr, qv, int(a.dim), g8);
             const float d = metric_from_sum(a.metric, sum);
-            const uint64_t e = (uint64_t(fkey(d)) << 32) | rrow;
-            // Insert the (up to) four new entries one after another.
-            for (int gg = 0; gg < 4; ++gg) {
-                if (r + uint32_t(gg) >= np) break;
-                const uint64_t x = __shfl_sync(kFull, e, gg * 8);
-                if (size >= kk && !entry_less(x, L[size - 1], a.keys)) continue;
-                list_insert(L, size, x, a.keys);
-                size = min(size + 1, kk);
-            }
+            const uint64_t e = brute_entry(a, d, rrow);
+            const uint64_t worst = t.n == kk ? t.L[kk - 1] : ~0ull;
+            const uint32_t W = __ballot_sync(kFull, g8 == 0 && slot < np && e < worst);
+            if (W) top_push(t, W, e, kk);
         }
         __syncwarp();
     }
+    if (t.cnt) top_flush(t, kk);
     const uint32_t want = min(a.k, a.n);
-    for (uint32_t i = lane; i < size && i < want; i += 32) {
-        a.out_keys[size_t(q) * a.k + i] = __ldg(a.keys + uint32_t(L[i]));
-        a.out_dist[size_t(q) * a.k + i] = kdec(uint32_t(L[i] >> 32));
+    for (uint32_t i = lane; i < t.n && i < want; i += 32) {
+        a.out_keys[size_t(q) * a.k + i] = __ldg(a.skeys + uint32_t(t.L[i]));
+        a.out_dist[size_t(q) * a.k + i] = kdec(uint32_t(t.L[i] >> 32));
     }
-    if (lane == 0) a.out_count[q] = min(size, want);
+    if (lane == 0) a.out_count[q] = min(t.n, want);
 }
 
 }  // namespace dev
@@ -365,38 +641,126 @@ cudaError_t launch_brute_rerank(const BruteArgs& a, const uint64_t* cand, const 
                                 const float* thr2, cudaStream_t stream) {
     const uint32_t kk = std::max<uint32_t>(1, std::min<uint32_t>(a.k, a.n ? a.n : 1));
     const uint32_t wpb = 4;
-    const size_t smem = size_t(wpb) * (kk + 1) * 8 + size_t(wpb) * 32 * 4;
+    const size_t smem = size_t(wpb) * (kk + 32) * 8 + size_t(wpb) * 32 * 4;
     cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(dev::brute_rerank_kernel));
     if (e != cudaSuccess) return e;
     dev::brute_rerank_kernel<<<(a.nq + wpb - 1) / wpb, 32 * wpb, smem, stream>>>(a, cand, cand_count, cand_cap, thr2, kk);
     return cudaGetLastError();
 }
 
+namespace {
+
+// The score kernel's shapes. A warp of eight queries x eight rows is the
+// general one; batches of one or two queries take QW = 2 so that the padding
+// is not computed, and small batches put more of the block's warps on rows.
+using TilePair = dev::BruteTile<2, 32, 1, 4>;
+using TileSmall = dev::BruteTile<8, 8, 1, 4>;
+using TileMid = dev::BruteTile<8, 8, 2, 2>;
+using TileBatch = dev::BruteTile<8, 8, 4, 1>;
+using TileLong = dev::BruteTile<8, 8, 1, 1>;  // lists in global memory (k above kSharedListMax)
+
+struct BrutePlan {
+    uint32_t qb = 0, rb = 0, threads = 0, slices = 0, kk = 0;
+    size_t smem = 0;
+    const void* kern = nullptr;  // null: no shape fits
+};
+
+constexpr size_t kBruteSmemMax = 227 * 1024;
+
+template <class T>
+bool take_tile(BrutePlan& p, uint32_t dp, uint32_t list_kk, bool l2) {
+    const size_t s = T::smem(dp, list_kk);
+    if (s > kBruteSmemMax) return false;
+    p.qb = T::QB;
+    p.rb = T::RB;
+    p.threads = T::kThreads;
+    p.smem = s;
+    p.kern = l2 ? reinterpret_cast<const void*>(dev::brute_score_kernel<true, T>)
+                : reinterpret_cast<const void*>(dev::brute_score_kernel<false, T>);
+    return true;
+}
+
+// Shape and row slices of a batch; at most max_slices lists per query.
+cudaError_t plan_brute(uint32_t nq, uint32_t n, uint32_t dp, uint32_t k, int metric, int num_sms, uint32_t max_slices,
+                       BrutePlan* out) {
+    BrutePlan p;
+    p.kk = std::max<uint32_t>(1, std::min<uint32_t>(k, n ? n : 1));
+    *out = p;
+    // Dimensions and k up to 24 rows and 16 lists of k + 1 entries in one
+    // block's shared memory are supported.
+    if (size_t(24) * dp * 4 + size_t(16) * (p.kk + 1) * 8 > kBruteSmemMax) return cudaErrorInvalidValue;
+    const bool l2 = metric == 0;
+    bool ok = false;
+    if (p.kk <= dev::kSharedListMax) {
+        if (nq <= 2) ok = take_tile<TilePair>(p, dp, p.kk, l2);
+        if (!ok && nq > 16) ok = take_tile<TileBatch>(p, dp, p.kk, l2);
+        if (!ok && nq > 8) ok = take_tile<TileMid>(p, dp, p.kk, l2);
+        if (!ok) ok = take_tile<TileSmall>(p, dp, p.kk, l2);
+    } else {
+        ok = take_tile<TileLong>(p, dp, 0, l2);
+    }
+    if (!ok) return cudaErrorInvalidValue;
+    cudaError_t e = raise_smem_limit(p.kern);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kern, int(p.threads), p.smem);
+    if (e != cudaSuccess) return e;
+    // Row slices: one full round of resident blocks (several when the query
+    // blocks alone come near one), fewer when a slice would fall below one
+    // row tile.
+    const uint64_t resident = uint64_t(num_sms) * uint64_t(std::max(per_sm, 1));
+    const uint64_t qblocks = (nq + p.qb - 1) / p.qb;
+    uint64_t s = qblocks >= resident ? (qblocks >= 4 * resident ? 1 : 4 * resident / qblocks) : resident / qblocks;
+    s = std::min<uint64_t>(s, (uint64_t(n) + p.rb - 1) / p.rb);
+    s = std::min<uint64_t>(std::min<uint64_t>(s, max_slices), 65535);
+    p.slices = uint32_t(std::max<uint64_t>(s, 1));
+    *out = p;
+    return cudaSuccess;
+}
+
+int current_sms() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 148;
+    return sms;
+}
+
+}  // namespace
+
+cudaError_t brute_slices(uint32_t nq, uint32_t n, uint32_t dp, uint32_t k, int metric, uint32_t* slices) {
+    BrutePlan p;
+    cudaError_t e = plan_brute(nq, n, dp, k, metric, current_sms(), ~0u, &p);
+    *slices = std::max<uint32_t>(p.slices, 1);
+    return e;
+}
+
 cudaError_t launch_brute_fp32(const BruteArgs& a, cudaStream_t stream) {
-    const uint32_t kk = std::max<uint32_t>(1, std::min<uint32_t>(a.k, a.n ? a.n : 1));
-    const uint32_t nslices = std::min<uint32_t>(a.tiles, 64);
+    const bool empty = a.n == 0 || a.k == 0;
+    BrutePlan p;
+    if (empty) p.kk = p.slices = 1;
+    else {
+        cudaError_t e = plan_brute(a.nq, a.n, a.dp, a.k, a.metric, current_sms(), a.tiles, &p);
+        if (e != cudaSuccess) return e;
+    }
     dev::brute_prep_kernel<<<(a.nq * 32 + 127) / 128, 128, 0, stream>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (a.n == 0 || a.k == 0) {
+    if (!empty) {
+        uint32_t rows_per = ((a.n + p.slices - 1) / p.slices + p.rb - 1) / p.rb * p.rb;
+        p.slices = (a.n + rows_per - 1) / rows_per;
         BruteArgs b = a;
-        dev::brute_merge_kernel<<<(a.nq * 32 + 127) / 128, 128, 0, stream>>>(b, kk, nslices);
-        return cudaGetLastError();
-    }
-    const size_t smem = (size_t(dev::kQB) + dev::kRT) * a.dp * 4 + size_t(dev::kQB) * (kk + 1) * 8;
-    dim3 grid((a.nq + dev::kQB - 1) / dev::kQB, nslices);
-    if (a.metric == 0) {
-        e = raise_smem_limit(reinterpret_cast<const void*>(dev::brute_score_kernel<true>));
+        void* argv[] = {&b, &p.kk, &rows_per, &p.slices};
+        e = cudaLaunchKernel(p.kern, dim3((a.nq + p.qb - 1) / p.qb, p.slices), dim3(p.threads), argv, p.smem, stream);
         if (e != cudaSuccess) return e;
-        dev::brute_score_kernel<true><<<grid, 128, smem, stream>>>(a, kk);
-    } else {
-        e = raise_smem_limit(reinterpret_cast<const void*>(dev::brute_score_kernel<false>));
-        if (e != cudaSuccess) return e;
-        dev::brute_score_kernel<false><<<grid, 128, smem, stream>>>(a, kk);
     }
-    e = cudaGetLastError();
+    // Warps of the merge: about 512 entries each, at most eight.
+    const uint64_t entries = uint64_t(p.slices) * p.kk;
+    const uint32_t nw = entries >= 4096 ? 8 : (entries >= 1024 ? 4 : (entries >= 512 ? 2 : 1));
+    const size_t smem = size_t(nw) * (p.kk + 32) * 8 + nw * 4;
+    e = raise_smem_limit(reinterpret_cast<const void*>(dev::brute_merge_kernel));
     if (e != cudaSuccess) return e;
-    dev::brute_merge_kernel<<<(a.nq * 32 + 127) / 128, 128, 0, stream>>>(a, kk, nslices);
+    dev::brute_merge_kernel<<<a.nq, 32 * nw, smem, stream>>>(a, p.kk, p.slices);
     return cudaGetLastError();
 }
 

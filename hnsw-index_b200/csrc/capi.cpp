@@ -1085,11 +1085,21 @@ int hnsw_gpu_brute_open(const float* vectors, const uint64_t* keys, size_t n, si
     }
     std::vector<uint64_t> kv(std::max<size_t>(n, 1));
     for (size_t i = 0; i < n; ++i) kv[i] = keys ? keys[i] : uint64_t(i);
-    if (keys) {
-        std::vector<uint64_t> sorted(kv.begin(), kv.begin() + n);
-        std::sort(sorted.begin(), sorted.end());
-        auto it = std::adjacent_find(sorted.begin(), sorted.end());
-        if (it != sorted.end()) return set_error(HNSW_ERR_DUPLICATE_KEY, "key " + std::to_string(*it) + " is already present");
+    // Keys that do not ascend are ranked: the kernels order ties by rank.
+    std::vector<uint64_t> sorted;
+    std::vector<uint32_t> rank;
+    if (keys && std::adjacent_find(kv.begin(), kv.begin() + n, std::greater_equal<uint64_t>()) != kv.begin() + n) {
+        std::vector<std::pair<uint64_t, uint32_t>> order(n);
+        for (size_t i = 0; i < n; ++i) order[i] = {kv[i], uint32_t(i)};
+        std::sort(order.begin(), order.end());
+        sorted.resize(n);
+        rank.resize(n);
+        for (size_t i = 0; i < n; ++i) {
+            sorted[i] = order[i].first;
+            rank[order[i].second] = uint32_t(i);
+            if (i && sorted[i] == sorted[i - 1])
+                return set_error(HNSW_ERR_DUPLICATE_KEY, "key " + std::to_string(sorted[i]) + " is already present");
+        }
     }
     DeviceGuard dg(device);
     std::unique_ptr<hnsw_gpu_brute> b(new hnsw_gpu_brute());
@@ -1112,6 +1122,12 @@ int hnsw_gpu_brute_open(const float* vectors, const uint64_t* keys, size_t n, si
     CU(cudaMemcpy(b->base.p, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice), "copy base");
     CU(b->keys.ensure(kv.size() * 8), "cudaMalloc keys");
     CU(cudaMemcpy(b->keys.p, kv.data(), kv.size() * 8, cudaMemcpyHostToDevice), "copy keys");
+    if (!rank.empty()) {
+        CU(b->krank.ensure(rank.size() * 4), "cudaMalloc key ranks");
+        CU(cudaMemcpy(b->krank.p, rank.data(), rank.size() * 4, cudaMemcpyHostToDevice), "copy key ranks");
+        CU(b->skeys.ensure(sorted.size() * 8), "cudaMalloc sorted keys");
+        CU(cudaMemcpy(b->skeys.p, sorted.data(), sorted.size() * 8, cudaMemcpyHostToDevice), "copy sorted keys");
+    }
     CU(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream");
     *out = b.release();
     return HNSW_OK;
@@ -1155,6 +1171,8 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     BruteArgs a;
     a.base = b->base.as<float>();
     a.keys = b->keys.as<uint64_t>();
+    a.krank = b->krank.as<uint32_t>();
+    a.skeys = b->skeys.p ? b->skeys.as<uint64_t>() : a.keys;
     a.n = b->n;
     a.dim = b->dim;
     a.dp = b->dp;
@@ -1301,17 +1319,22 @@ static int brute_search_fp32(hnsw_gpu_brute* b, const float* queries, size_t nq,
     BruteArgs a;
     a.base = b->base.as<float>();
     a.keys = b->keys.as<uint64_t>();
+    a.krank = b->krank.as<uint32_t>();
+    a.skeys = b->skeys.p ? b->skeys.as<uint64_t>() : a.keys;
     a.n = b->n;
     a.dim = b->dim;
     a.dp = b->dp;
     a.metric = b->metric;
     a.nq = uint32_t(nq);
     a.k = k;
-    a.tiles = std::max<uint32_t>(1, std::min<uint32_t>(64, (b->n + 8191) / 8192));
+    a.tiles = 1;
+    if (b->n && k) CU(brute_slices(a.nq, b->n, b->dp, k, b->metric, &a.tiles), "brute kernel");
     CU(b->q.ensure(nq * dim * 4), "cudaMalloc queries");
     CU(cudaMemcpyAsync(b->q.p, queries, nq * dim * 4, cudaMemcpyHostToDevice, st), "copy queries");
     CU(b->qprep.ensure(nq * b->dp * 4), "cudaMalloc qprep");
     CU(b->part.ensure(size_t(nq) * a.tiles * kk * 8), "cudaMalloc partial");
+    CU(b->minima.ensure(nq * kBruteMinima * 4), "cudaMalloc lane minima");
+    a.minima = b->minima.as<uint32_t>();
     CU(b->okeys.ensure(nq * kk * 8), "cudaMalloc out keys");
     CU(b->odist.ensure(nq * kk * 4), "cudaMalloc out dist");
     CU(b->ocount.ensure(nq * 4), "cudaMalloc out count");
@@ -1454,16 +1477,22 @@ int hnsw_gpu_brute_search_batch_noalloc(hnsw_gpu_brute* b, const float* d_querie
     void* scratch = nullptr;
     CU(noalloc_scratch_address(&scratch), "no-alloc scratch address");
     const uint32_t kk = std::max<uint32_t>(1, std::min<uint32_t>(k, b->n ? b->n : 1));
-    const uint32_t want = std::max<uint32_t>(1, std::min<uint32_t>(64, (b->n + 8191) / 8192));
+    uint32_t want = 1;
     size_t qbytes = 0;
     uint32_t slices = 0;
     if (!noalloc_layout(uint32_t(nq), b->dp, kk, want, &qbytes, &slices))
         return set_error(HNSW_ERR_INVALID_ARGUMENT,
                          "batch too large for the no-alloc scratch: round_up(nq * 4 * round_up(dim, 32), 256) + "
                          "nq * 8 * max(1, min(k, n)) must not exceed 8 MiB");
+    if (b->n && k) {
+        CU(brute_slices(uint32_t(nq), b->n, b->dp, k, b->metric, &want), "brute kernel (no-alloc)");
+        noalloc_layout(uint32_t(nq), b->dp, kk, want, &qbytes, &slices);
+    }
     BruteArgs a;
     a.base = b->base.as<float>();
     a.keys = b->keys.as<uint64_t>();
+    a.krank = b->krank.as<uint32_t>();
+    a.skeys = b->skeys.p ? b->skeys.as<uint64_t>() : a.keys;
     a.n = b->n;
     a.dim = b->dim;
     a.dp = b->dp;

@@ -214,9 +214,10 @@ struct hnsw_gpu_brute {
     int metric = 0;
     float max_xnorm = 0.0f;  // largest row norm (error margins of the tensor-core path)
     DBuf base, keys;
+    DBuf krank, skeys;  // key ranks and sorted keys, when the keys do not ascend
     SlotPool slots;
     std::mutex mu;
-    DBuf qprep, part, okeys, odist, ocount, ostatus, q;
+    DBuf qprep, part, minima, okeys, odist, ocount, ostatus, q;
     DBuf fbits, fused, fids;  // filter bitmaps, flags and bitmap ids of a filtered search
     // Tensor-core path: BF16 operand rows per term count (index 0: 1 term, 1: 3 terms).
     DBuf bop[2], xnorm2;
@@ -231,7 +232,7 @@ struct hnsw_gpu_brute {
     cudaStream_t stream = nullptr;
     ~hnsw_gpu_brute() {
         DeviceGuard g(device);
-        for (DBuf* b : {&base, &keys, &qprep, &part, &okeys, &odist, &ocount, &ostatus, &q, &fbits, &fused, &fids,
+        for (DBuf* b : {&base, &keys, &krank, &skeys, &qprep, &part, &minima, &okeys, &odist, &ocount, &ostatus, &q, &fbits, &fused, &fids,
                         &bop[0], &bop[1], &xnorm2,
                         &aop, &dense, &thr1, &thr2, &margin, &qnorm2, &ccount, &cand, &err})
             b->release();

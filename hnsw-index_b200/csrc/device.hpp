@@ -223,11 +223,18 @@ cudaError_t launch_encode_codes(const float* vec, uint32_t n, uint32_t dim, uint
                                 const float* offset, float scale, int8_t* codes, int32_t* norms,
                                 cudaStream_t stream);
 
+constexpr uint32_t kBruteMinima = 128;  // lane minima kept per query
+
 // Exact FP32 brute force in the reference kernel order (K1 per row) with a
 // per-query top-k merge.
 struct BruteArgs {
     const float* base = nullptr;  // n * dp, prepared
     const uint64_t* keys = nullptr;
+    // Ties are broken by key: krank[row] is the rank of the row's key and
+    // skeys the keys in ascending order (krank null, skeys = keys, when the
+    // rows' keys ascend).
+    const uint32_t* krank = nullptr;
+    const uint64_t* skeys = nullptr;
     uint32_t n = 0, dim = 0, dp = 0;
     int metric = 0;
     const float* queries = nullptr;  // nq * dim raw
@@ -238,8 +245,9 @@ struct BruteArgs {
     int32_t* out_status = nullptr;
     // scratch
     float* qprep = nullptr;         // nq * dp
-    uint64_t* part = nullptr;       // nq * tiles * k partial top-k (packed dist key, row)
-    uint32_t tiles = 0;
+    uint64_t* part = nullptr;       // nq * tiles * k partial top-k (packed dist key, key rank)
+    uint32_t tiles = 0;             // lists per query `part` has room for
+    uint32_t* minima = nullptr;     // optional, nq * kBruteMinima: smallest distances of some lanes (bounds)
     // Optional filter (BruteForceIndex::search_filtered): a row is scored
     // only when its bit is set; bit = key, or row index with filter_by_row.
     // Query q uses bitmap filter_ids[q] (or q) at filter_stride words each
@@ -252,6 +260,9 @@ struct BruteArgs {
     int filter_by_row = 0;
 };
 cudaError_t launch_brute_fp32(const BruteArgs& a, cudaStream_t stream);
+// Row slices (lists per query) that a batch is cut into when nothing limits
+// them; launch_brute_fp32 uses at most a.tiles.
+cudaError_t brute_slices(uint32_t nq, uint32_t n, uint32_t dp, uint32_t k, int metric, uint32_t* slices);
 // Query preparation only (vector::check, cosine normalisation) into a.qprep.
 cudaError_t launch_brute_prep(const BruteArgs& a, cudaStream_t stream);
 // Exact FP32 re-rank of packed (approx distance bits << 32 | row) candidates
