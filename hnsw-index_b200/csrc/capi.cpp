@@ -205,6 +205,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     }
     if (o.mode == HNSW_MODE_AUTO) o.mode = HNSW_MODE_PERSISTENT;
     const bool persistent = o.mode == HNSW_MODE_PERSISTENT, filtered = d_fbits != nullptr;
+    const bool heuristic = !geo.ef_cap;
     if (!geo.ef_cap) geo = pick_geometry(ef_max, gi->view.dp, gi->view.dc, persistent, filtered, gi->view.n);
     geo.stage_row_bytes =
         geo.stage_rows ? ((o.quantized && gi->view.quantized) ? gi->view.dc : gi->view.dp * 4) : 0;
@@ -276,7 +277,27 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     a.overflow_count = s->work.as<uint32_t>() + 1;
     a.overflow_list = s->overflow.as<uint32_t>();
     a.persistent = o.mode == HNSW_MODE_PERSISTENT ? 1 : 0;
-    if (a.persistent) {
+    // A team of warps per query where one warp each would leave the batch
+    // waiting on memory latency: up to two teams per SM, or four when the
+    // queries are alike. Larger batches of unlike queries (filters, an ef per
+    // query) are decided on the device from their expected work.
+    TeamGeometry team;
+    const bool plans = o.exact_below > 0.0f && d_fbits, varied = d_efs || d_fbits;
+    const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
+    if (heuristic && !o.traversal && !plans && tags == 0 && (small || varied))
+        CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
+    if (team.blocks) {
+        // Without memory for the teams the batch takes the warp kernels.
+        const size_t row = team.bitmap_words ? 0 : ((size_t(gi->view.n) + 31) / 32 + 3) / 4 * 16;
+        cudaError_t e = s->team_far.ensure(size_t(team.blocks) * team.far_cap * 8);
+        if (e == cudaSuccess && row) e = s->team_bits.ensure(size_t(team.blocks) * row);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            team = TeamGeometry();
+        }
+    }
+    const bool warp_route = !team.blocks || !small;
+    if (a.persistent && warp_route) {
         uint32_t warps = 0;
         CU(persistent_warps(geo, gi->view.dp, gi->view.dc, gi->num_sms, &warps), "occupancy");
         const uint32_t words = ((gi->view.n + 31) / 32 + 3) & ~3u;
@@ -294,6 +315,17 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         a.spill_bits = s->spill_bits.as<uint32_t>();
         a.spill_words = words;
         a.spill_slots = warps;
+    }
+    if (!warp_route) geo.cold = 0;
+    if (team.blocks && varied && nq > team.blocks) {
+        CU(s->order.ensure(nq * 5), "cudaMalloc query order");
+        const uint32_t slots = a.persistent && warp_route ? a.spill_slots : uint32_t(gi->num_sms) * 16;
+        uint32_t* route = s->work.as<uint32_t>() + 5;
+        CU(launch_query_order(a, s->order.as<uint32_t>(), s->order.as<uint8_t>() + nq * 4, slots, team.blocks, route,
+                              stream),
+           "query order");
+        a.order = s->order.as<uint32_t>();
+        if (warp_route) a.route = route;
     }
     // Cold candidate lists (the cold variant's persistent warps, then the
     // retry warps, which reuse the whole pool): 8 entries per node or 32
@@ -332,13 +364,22 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     }
     a.overflow_list2 = s->overflow2.as<uint32_t>();
     a.overflow_count2 = s->work.as<uint32_t>() + 4;
-    if (o.exact_below > 0.0f && d_fbits) {
+    if (plans) {
         CU(s->planned.ensure(std::max<size_t>(nq, 1)), "cudaMalloc planner flags");
         a.plan_max = uint32_t(std::max(1.0, std::floor(double(o.exact_below) * double(gi->view.live))));
         CU(launch_plan(a, s->planned.as<uint8_t>(), stream), "planner kernel");
         a.planned = s->planned.as<uint8_t>();
     }
-    CU(launch_search(a, geo, gi->num_sms, stream), "search kernel");
+    if (warp_route) CU(launch_search(a, geo, gi->num_sms, stream), "search kernel");
+    if (team.blocks) {
+        SearchArgs ta = a;
+        if (!team.bitmap_words) {
+            ta.spill_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
+            ta.spill_bits = s->team_bits.as<uint32_t>();
+        }
+        ta.team_far = s->team_far.as<uint64_t>();
+        CU(launch_search_team(ta, team, stream), "search team kernel");
+    }
     CU(launch_search_retry(a, s->g_warps, stream), "search retry kernel");
     SearchArgs last = a;
     last.overflow_list = a.overflow_list2;

@@ -84,11 +84,12 @@ struct Slot {
     DBuf cold_pool, cold_tab; // cold candidate lists (persistent and retry warps)
     DBuf last_pool, last_tab, overflow2;  // last-resort pass (private cold regions)
     DBuf planned;                         // selectivity planner flags
+    DBuf team_bits, team_far, order;      // team traversal: visited bitmaps, far candidates, query order
     size_t last_nq = 0;
     ~Slot() {
         for (DBuf* b : {&q, &ks, &efs, &fbits, &fused, &fids, &okeys, &odist, &ocount, &ostatus, &work, &overflow, &counters,
                         &g_results, &g_cands, &g_visited, &spill_bits, &spill_cands, &cold_pool, &cold_tab, &last_pool,
-                        &last_tab, &overflow2, &planned})
+                        &last_tab, &overflow2, &planned, &team_bits, &team_far, &order})
             b->release();
         if (stream) cudaStreamDestroy(stream);
     }

@@ -114,6 +114,11 @@ struct SearchArgs {
     uint32_t* overflow_list = nullptr;
     uint32_t* overflow_count = nullptr;
     int persistent = 0;
+    uint64_t* team_far = nullptr;     // team kernel: far candidates, far_cap per block
+    // Query of each work counter value (null: the same), and the kernel that
+    // takes the batch when the device decides (null: the one launched).
+    const uint32_t* order = nullptr;
+    const uint32_t* route = nullptr;
     // Fallback workspaces in global memory (retry kernel only).
     uint64_t* g_results = nullptr;
     uint64_t* g_cands = nullptr;
@@ -178,6 +183,26 @@ __host__ __device__ inline uint32_t tc_query_bytes(const SearchArgs& a) {
 }
 
 constexpr uint32_t kLastResortWarps = 4;
+
+// Team traversal (search_team.cu): a block of warps per query. blocks == 0:
+// the batch cannot take it.
+struct TeamGeometry {
+    uint32_t ef_cap = 0, cand_cap = 0;
+    uint32_t warps = 0;         // per team: 4 or 8
+    uint32_t far_cap = 0;       // entries of a block's far list (args.team_far)
+    uint32_t bitmap_words = 0;  // visited bitmap in shared memory; 0: in args.spill_bits, one row per block
+    uint32_t blocks = 0;
+    size_t smem = 0;
+};
+// Geometry for args.nq queries whose max(ef, k) is at most ef_max.
+cudaError_t plan_search_team(const SearchArgs& args, uint32_t ef_max, int num_sms, TeamGeometry* out);
+cudaError_t launch_search_team(const SearchArgs& args, const TeamGeometry& geo, cudaStream_t stream);
+// Query indices in descending order of expected work, and the kernel to take
+// the batch (kRoute*) given the warps or teams resident at once; `bucket` is
+// scratch (nq bytes).
+constexpr uint32_t kRouteWarp = 1, kRouteTeam = 2;
+cudaError_t launch_query_order(const SearchArgs& args, uint32_t* order, uint8_t* bucket, uint32_t warp_slots,
+                               uint32_t team_slots, uint32_t* route, cudaStream_t stream);
 
 constexpr uint32_t kColdChunkShift = 10;
 constexpr uint32_t kColdChunk = 1u << kColdChunkShift;  // entries per cold chunk (8 KB)

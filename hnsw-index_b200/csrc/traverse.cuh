@@ -1250,13 +1250,16 @@ static __device__ int32_t prepare(QueryCtx& c, const float* q) {
     bad = __any_sync(kFull, bad);
     __syncwarp();
     if (bad) return ST_NON_FINITE;
+    // The f64 sum adds its terms in row order; the products are formed 32 at
+    // a time, one per lane, so that only the additions are serial.
     double norm = 0.0;
-    if (lane == 0)
-        for (uint32_t i = 0; i < dim; ++i) {
-            double x = double(w.qf[i]);
-            norm = __dadd_rn(norm, __dmul_rn(x, x));
-        }
-    norm = __shfl_sync(kFull, norm, 0);
+    for (uint32_t b = 0; b < dim; b += 32) {
+        const double x = double(w.qf[b + lane]);
+        const double p = __dmul_rn(x, x);
+        const uint32_t m = min(32u, dim - b);
+#pragma unroll 8
+        for (uint32_t j = 0; j < m; ++j) norm = __dadd_rn(norm, __shfl_sync(kFull, p, int(j)));
+    }
     if (norm > double(3.40282346638528859812e+38F) / 8.0) return ST_NON_FINITE;  // f32::MAX / 8
     if (c.metric == 2) {
         if (norm == 0.0) return ST_ZERO;
@@ -1513,6 +1516,7 @@ static __device__ void end_spill(Ws& w) {
 template <int V, int DK = DK_ANY, bool PERSIST = false>
 __global__ void __launch_bounds__(256, 2) search_kernel(SearchArgs a, SearchGeometry g) {
     extern __shared__ __align__(16) char smem[];
+    if (a.route && *a.route != kRouteWarp) return;
     const uint32_t warp = threadIdx.x >> 5;
     Ws w;
     carve(w, smem + size_t(warp) * g.bytes_per_warp, a.ix, g);
@@ -1536,6 +1540,7 @@ __global__ void __launch_bounds__(256, 2) search_kernel(SearchArgs a, SearchGeom
             if (lane == 0) qi = atomicAdd(a.work_next, 1u);
             qi = __shfl_sync(kFull, qi, 0);
             if (qi >= a.nq) break;
+            if (a.order) qi = __ldg(a.order + qi);
             const int32_t st = run_query<V, DK>(a, w, qi, qi);
             end_spill(w);
             if (st == ST_OVERFLOW && lane == 0) {

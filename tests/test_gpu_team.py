@@ -1,0 +1,88 @@
+"""Team traversal (a block of warps per query) against the oracle: batches at
+the edges of its rule (one query, two teams per SM, four per SM, one more), all
+metrics and row kinds, lists of one and two 32-id chunks, walks that fill the
+queue's far list, equal distances everywhere (small integers), deleted nodes,
+a visited bitmap in global memory, and batches routed on the device. Keys,
+distance bits, counts and statuses are equal (no tolerance)."""
+
+import numpy as np
+import pytest
+
+import hnsw_gpu as H
+import oracle as O
+from conftest import build_index
+
+pytestmark = pytest.mark.gpu
+
+
+def assert_same(got, ref, what):
+    np.testing.assert_array_equal(got[3], ref[3], err_msg=what)
+    np.testing.assert_array_equal(got[2], ref[2], err_msg=what)
+    for i in range(len(got[2])):
+        c = int(got[2][i])
+        np.testing.assert_array_equal(got[0][i, :c], ref[0][i, :c], err_msg=f"{what} query {i}")
+        np.testing.assert_array_equal(got[1][i, :c].view(np.uint32), ref[1][i, :c].view(np.uint32), err_msg=what)
+
+
+@pytest.mark.parametrize("metric", [0, 1, 2])
+@pytest.mark.parametrize("dim,m,n", [(8, 4, 300), (100, 16, 4000), (40, 24, 3000), (33, 40, 2000)])
+def test_team_walks(metric, dim, m, n):
+    base, q = H.mixture(n, 300, dim, 20, 0.4, metric * 7 + dim)
+    if dim == 8:  # ties
+        base, q = np.round(base * 2), np.round(q * 2)
+        base[:, 0] += 10
+        q[:, 0] += 10
+    if metric == 2:
+        base[:, 0] += 2
+        q[:, 0] += 2
+    rng = np.random.default_rng(n + metric)
+    deleted = rng.choice(n, n // 20, replace=False) if dim != 100 else ()
+    data = build_index(base, metric=metric, m=m, ef_construction=60, quantize=True, deleted_keys=deleted)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    for nq, k, ef in ((1, 1, 1), (3, 10, 16), (296, 10, 64), (200, 100, 300)):
+        what = f"nq={nq} k={k} ef={ef}"
+        assert_same(gi.search_arrays(q[:nq], k, ef), oi.search(q[:nq], k, ef), what)
+        assert_same(gi.search_arrays(q[:nq], k, ef, quantized=True, mode=1),
+                    oi.search(q[:nq], k, ef, quantized=True), what + " int8")
+        for sel in (0.01, 0.2):
+            bits = H.key_bitmap(np.nonzero(rng.random(n) < sel)[0].astype(np.uint64), n)
+            kw = dict(filter_bits=bits, filter_nbits=n)
+            assert_same(gi.search_arrays(q[:nq], k, ef, mode=nq & 1, **kw), oi.search(q[:nq], k, ef, **kw),
+                        what + f" filter {sel}")
+
+
+@pytest.mark.parametrize("nq", [297, 592, 593])
+def test_team_batches_around_the_rule(nq):
+    base, q = H.gaussian(5000, 593, 32, 3)
+    data = build_index(base, ef_construction=60)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    assert_same(gi.search_arrays(q[:nq], 10, 48), oi.search(q[:nq], 10, 48), f"nq={nq}")
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("sel", [0.02, 0.9])
+def test_batches_routed_on_the_device(mode, sel):
+    """Few long walks among short ones, and walks of like length."""
+    n, nq = 6000, 900
+    base, q = H.mixture(n, nq, 24, 30, 0.4, 5)
+    data = build_index(base, metric=1, ef_construction=60, quantize=True)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    rng = np.random.default_rng(8)
+    bits = H.key_bitmap(np.nonzero(rng.random(n) < sel)[0].astype(np.uint64), n)
+    used = (np.arange(nq) % 50 == 0).astype(np.uint8) if sel < 0.1 else np.ones(nq, np.uint8)
+    ks, efs = rng.choice([1, 10, 50], nq).astype(np.uint32), rng.choice([16, 64, 128], nq).astype(np.uint32)
+    kw = dict(filter_bits=bits, filter_nbits=n, filter_used=used, ks=ks, efs=efs, quantized=True)
+    assert_same(gi.search_arrays(q, 10, 16, mode=mode, **kw), oi.search(q, 10, 16, **kw), f"mode={mode} sel={sel}")
+
+
+def test_team_with_its_visited_bitmap_in_global_memory():
+    n = 800_000
+    base, q = H.mixture(n, 160, 4, 500, 0.3, 2)
+    b = H.IndexBuilder(4, H.Metric.L2, H.HnswParams(m=4, ef_construction=16, seed=7))
+    b.insert_batch_gpu(np.arange(n, dtype=np.uint64), base)
+    data = b.to_bytes()
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    assert_same(gi.search_arrays(q, 10, 40), oi.search(q, 10, 40), "plain")
+    bits = H.key_bitmap(np.arange(0, n, 3, dtype=np.uint64), n)
+    kw = dict(filter_bits=bits, filter_nbits=n)
+    assert_same(gi.search_arrays(q, 10, 40, **kw), oi.search(q, 10, 40, **kw), "filtered")
