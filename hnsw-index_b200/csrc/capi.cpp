@@ -206,7 +206,17 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     if (o.mode == HNSW_MODE_AUTO) o.mode = HNSW_MODE_PERSISTENT;
     const bool persistent = o.mode == HNSW_MODE_PERSISTENT, filtered = d_fbits != nullptr;
     const bool heuristic = !geo.ef_cap;
-    if (!geo.ef_cap) geo = pick_geometry(ef_max, gi->view.dp, gi->view.dc, persistent, filtered, gi->view.n);
+    if (heuristic) {
+        const uint64_t key = uint64_t(std::min<uint32_t>(1024, std::max<uint32_t>(32, round_up(ef_max, 32)))) |
+                             uint64_t(persistent) << 32 | uint64_t(filtered) << 33 |
+                             uint64_t(g_visit_tag_bits.load() + 1) << 34;
+        std::lock_guard<std::mutex> l(gi->plan_mu);
+        auto it = gi->plans.find(key);
+        if (it == gi->plans.end())
+            it = gi->plans.emplace(key, pick_geometry(ef_max, gi->view.dp, gi->view.dc, persistent, filtered, gi->view.n))
+                     .first;
+        geo = it->second;
+    }
     geo.stage_row_bytes =
         geo.stage_rows ? ((o.quantized && gi->view.quantized) ? gi->view.dc : gi->view.dp * 4) : 0;
     geo.tc_bytes = tcb;
@@ -755,10 +765,7 @@ static int stage_batch(Slot* s, const float* queries, size_t nq, size_t dim, con
             d_fu = s->fused.as<uint8_t>();
         }
     }
-    CU(s->okeys.ensure(nq * stride * 8), "cudaMalloc out keys");
-    CU(s->odist.ensure(nq * stride * 4), "cudaMalloc out dist");
-    CU(s->ocount.ensure(nq * 4), "cudaMalloc out count");
-    CU(s->ostatus.ensure(nq * 4), "cudaMalloc out status");
+    CU(s->out.ensure(nq, stride), "cudaMalloc outputs");
     out->ks = d_ks;
     out->efs = d_efs;
     out->fbits = d_fb;
@@ -805,14 +812,9 @@ int hnsw_gpu_search_batch(hnsw_gpu_index* gi, const float* queries, size_t nq, s
     r = stage_batch(s, queries, nq, dim, o, stride, &sb);
     if (r != HNSW_OK) return r;
     r = enqueue_search(gi, s, s->q.as<float>(), nq, o, sb.ks, sb.efs, sb.fbits, sb.fused, sb.fids,
-                       s->okeys.as<uint64_t>(), s->odist.as<float>(), s->ocount.as<uint32_t>(),
-                       s->ostatus.as<int32_t>(), ef_bound, stride, st);
+                       s->out.keys(), s->out.dist(), s->out.count(), s->out.status(), ef_bound, stride, st);
     if (r != HNSW_OK) return r;
-    CU(cudaMemcpyAsync(out_count, s->ocount.p, nq * 4, cudaMemcpyDeviceToHost, st), "copy counts");
-    CU(cudaMemcpyAsync(out_status, s->ostatus.p, nq * 4, cudaMemcpyDeviceToHost, st), "copy statuses");
-    CU(cudaMemcpyAsync(out_keys, s->okeys.p, nq * stride * 8, cudaMemcpyDeviceToHost, st), "copy keys");
-    CU(cudaMemcpyAsync(out_dist, s->odist.p, nq * stride * 4, cudaMemcpyDeviceToHost, st), "copy distances");
-    CU(cudaStreamSynchronize(st), "search");
+    CU(s->out.fetch(st, out_keys, out_dist, out_count, out_status), "search");
     if (gi->counters) {
         std::lock_guard<std::mutex> g(gi->counters_mu);
         gi->last_counters.resize(nq * 4);
@@ -886,8 +888,8 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
         ot.mode = mode;
         auto run = [&]() {
             return enqueue_search(gi, s, s->q.as<float>(), nq, ot, sb.ks, sb.efs, sb.fbits, sb.fused, sb.fids,
-                                  s->okeys.as<uint64_t>(), s->odist.as<float>(), s->ocount.as<uint32_t>(),
-                                  s->ostatus.as<int32_t>(), ef_bound, stride, st, &g);
+                                  s->out.keys(), s->out.dist(), s->out.count(), s->out.status(), ef_bound, stride, st,
+                                  &g);
         };
         r = run();  // warm-up; sizes every buffer
         if (r != HNSW_OK) return false;
@@ -1225,16 +1227,16 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     CU(b->q.ensure(nq * b->dim * 4), "cudaMalloc queries");
     CU(cudaMemcpyAsync(b->q.p, queries, nq * b->dim * 4, cudaMemcpyHostToDevice, st), "copy queries");
     CU(b->qprep.ensure(size_t(qp) * b->dp * 4), "cudaMalloc qprep");
-    CU(b->okeys.ensure(nq * size_t(k) * 8), "cudaMalloc out keys");
-    CU(b->odist.ensure(nq * size_t(k) * 4), "cudaMalloc out dist");
-    CU(b->ocount.ensure(nq * 4), "cudaMalloc out count");
-    CU(b->ostatus.ensure(nq * 4), "cudaMalloc out status");
+    // Beside the outputs: the candidate counts, and the error word after them.
+    CU(b->out.ensure(nq, k, (size_t(qp) + 1) * 4), "cudaMalloc outputs");
+    uint32_t* d_ccount = b->out.extra();
+    uint32_t* d_err = d_ccount + qp;
     a.queries = b->q.as<float>();
     a.qprep = b->qprep.as<float>();
-    a.out_keys = b->okeys.as<uint64_t>();
-    a.out_dist = b->odist.as<float>();
-    a.out_count = b->ocount.as<uint32_t>();
-    a.out_status = b->ostatus.as<int32_t>();
+    a.out_keys = b->out.keys();
+    a.out_dist = b->out.dist();
+    a.out_count = b->out.count();
+    a.out_status = b->out.status();
     CU(cudaEventRecord(b->ev[0], st), "event");
     CU(launch_brute_prep(a, st), "query prep");
     // Query norms (L2 epilogue and margins) and BF16 query operands.
@@ -1249,8 +1251,7 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     CU(tc_margins(b->qnorm2.as<float>(), uint32_t(nq), b->max_xnorm, float(eps), b->metric, b->dim,
                   b->margin.as<float>(), st),
        "margins");
-    CU(b->err.ensure(16), "cudaMalloc error word");
-    CU(cudaMemsetAsync(b->err.p, 0, 16, st), "memset error word");
+    CU(cudaMemsetAsync(d_ccount, 0, (size_t(qp) + 1) * 4, st), "memset candidate counts and error word");
     // Sample pass.
     CU(cudaEventRecord(b->ev[1], st), "event");
     const uint32_t sample_rows = std::min<uint32_t>(np, 16384);
@@ -1264,7 +1265,7 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     t.metric = b->metric;
     t.qnorm2 = b->qnorm2.as<float>();
     t.xnorm2 = b->metric == HNSW_METRIC_L2 ? b->xnorm2.as<float>() : nullptr;
-    t.err = b->err.as<uint32_t>();
+    t.err = d_err;
     t.wait_budget = b->wait_budget;
     t.stall = b->stall;
     t.pairs = pairs ? 1u : 0u;
@@ -1280,33 +1281,27 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
        "sample threshold");
     // Candidate pass.
     const uint32_t cap = 32768;
-    CU(b->ccount.ensure(size_t(qp) * 4), "cudaMalloc candidate counts");
     CU(b->cand.ensure(size_t(nq) * cap * 8), "cudaMalloc candidates");
-    CU(cudaMemsetAsync(b->ccount.p, 0, size_t(qp) * 4, st), "memset candidate counts");
     t.dense = nullptr;
     t.n_tile_begin = 0;
     t.n_tile_end = np / 256;
     t.thr = b->thr1.as<float>();
-    t.cand_count = b->ccount.as<uint32_t>();
+    t.cand_count = d_ccount;
     t.cand = b->cand.as<uint64_t>();
     t.cand_cap = cap;
     CU(cudaEventRecord(b->ev[2], st), "event");
     CU(tc_score(b->aop.as<__nv_bfloat16>(), qp, b->bop[ti].as<__nv_bfloat16>(), np, kp, t, b->num_sms, st),
        "candidate pass");
     CU(cudaEventRecord(b->ev[3], st), "event");
-    CU(tc_kth_threshold(nullptr, 0, b->ccount.as<uint32_t>(), b->cand.as<uint64_t>(), cap, uint32_t(nq), kk,
+    CU(tc_kth_threshold(nullptr, 0, d_ccount, b->cand.as<uint64_t>(), cap, uint32_t(nq), kk,
                         b->margin.as<float>(), b->thr2.as<float>(), st),
        "candidate threshold");
-    CU(launch_brute_rerank(a, b->cand.as<uint64_t>(), b->ccount.as<uint32_t>(), cap, b->thr2.as<float>(), st),
+    CU(launch_brute_rerank(a, b->cand.as<uint64_t>(), d_ccount, cap, b->thr2.as<float>(), st),
        "re-rank");
     CU(cudaEventRecord(b->ev[4], st), "event");
-    uint32_t err = 0;
-    CU(cudaMemcpyAsync(&err, b->err.p, 4, cudaMemcpyDeviceToHost, st), "copy error word");
-    CU(cudaMemcpyAsync(out_count, a.out_count, nq * 4, cudaMemcpyDeviceToHost, st), "copy counts");
-    CU(cudaMemcpyAsync(out_status, a.out_status, nq * 4, cudaMemcpyDeviceToHost, st), "copy statuses");
-    CU(cudaMemcpyAsync(out_keys, a.out_keys, nq * size_t(k) * 8, cudaMemcpyDeviceToHost, st), "copy keys");
-    CU(cudaMemcpyAsync(out_dist, a.out_dist, nq * size_t(k) * 4, cudaMemcpyDeviceToHost, st), "copy distances");
-    CU(cudaStreamSynchronize(st), "tensor brute force");
+    std::vector<uint32_t> extra(size_t(qp) + 1);
+    CU(b->out.fetch(st, out_keys, out_dist, out_count, out_status, true, extra.data()), "tensor brute force");
+    const uint32_t err = extra[qp];
     for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&b->last_ms[i], b->ev[i], b->ev[i + 1]);
     if (err) return set_error(HNSW_ERR_TIMEOUT, "tensor-core scoring: a bounded wait ran out");
     // Queries whose candidate list overflowed: exact FP32 kernels.
@@ -1334,15 +1329,9 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
             std::memcpy(out_dist + i * k, &sd[j * k], size_t(k) * 4);
         }
     }
-    {
-        std::vector<uint32_t> counts(nq);
-        if (cudaMemcpy(counts.data(), b->ccount.p, nq * 4, cudaMemcpyDeviceToHost) == cudaSuccess) {
-            uint64_t total = 0;
-            for (uint32_t c : counts) total += c;
-            b->last_candidates = total;
-            b->last_queries = nq;
-        }
-    }
+    b->last_candidates = 0;
+    for (size_t i = 0; i < nq; ++i) b->last_candidates += extra[i];
+    b->last_queries = nq;
     for (size_t i = 0; i < nq; ++i)
         if (out_status[i] != HNSW_OK) return set_error(out_status[i], "query failed validation");
     return HNSW_OK;
@@ -1376,17 +1365,14 @@ static int brute_search_fp32(hnsw_gpu_brute* b, const float* queries, size_t nq,
     CU(b->part.ensure(size_t(nq) * a.tiles * kk * 8), "cudaMalloc partial");
     CU(b->minima.ensure(nq * kBruteMinima * 4), "cudaMalloc lane minima");
     a.minima = b->minima.as<uint32_t>();
-    CU(b->okeys.ensure(nq * kk * 8), "cudaMalloc out keys");
-    CU(b->odist.ensure(nq * kk * 4), "cudaMalloc out dist");
-    CU(b->ocount.ensure(nq * 4), "cudaMalloc out count");
-    CU(b->ostatus.ensure(nq * 4), "cudaMalloc out status");
+    CU(b->out.ensure(nq, kk), "cudaMalloc outputs");
     a.queries = b->q.as<float>();
     a.qprep = b->qprep.as<float>();
     a.part = b->part.as<uint64_t>();
-    a.out_keys = b->okeys.as<uint64_t>();
-    a.out_dist = b->odist.as<float>();
-    a.out_count = b->ocount.as<uint32_t>();
-    a.out_status = b->ostatus.as<int32_t>();
+    a.out_keys = b->out.keys();
+    a.out_dist = b->out.dist();
+    a.out_count = b->out.count();
+    a.out_status = b->out.status();
     if (f && f->bits) {
         const uint64_t words = (f->nbits + 63) / 64;
         uint64_t bitmaps = f->stride ? nq : 1;
@@ -1412,13 +1398,7 @@ static int brute_search_fp32(hnsw_gpu_brute* b, const float* queries, size_t nq,
         }
     }
     CU(launch_brute_fp32(a, st), "brute kernel");
-    CU(cudaMemcpyAsync(out_count, b->ocount.p, nq * 4, cudaMemcpyDeviceToHost, st), "copy counts");
-    CU(cudaMemcpyAsync(out_status, b->ostatus.p, nq * 4, cudaMemcpyDeviceToHost, st), "copy statuses");
-    if (k) {
-        CU(cudaMemcpyAsync(out_keys, b->okeys.p, nq * size_t(k) * 8, cudaMemcpyDeviceToHost, st), "copy keys");
-        CU(cudaMemcpyAsync(out_dist, b->odist.p, nq * size_t(k) * 4, cudaMemcpyDeviceToHost, st), "copy distances");
-    }
-    CU(cudaStreamSynchronize(st), "brute search");
+    CU(b->out.fetch(st, out_keys, out_dist, out_count, out_status, k != 0), "brute search");
     for (size_t i = 0; i < nq; ++i)
         if (out_status[i] != HNSW_OK) return set_error(out_status[i], "query failed validation");
     return HNSW_OK;

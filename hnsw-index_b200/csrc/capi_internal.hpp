@@ -9,7 +9,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstring>
 #include <functional>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -73,10 +75,82 @@ struct DBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
+// The outputs of one host-buffer call in one device buffer, so that they come
+// back in one copy: keys and distances (nq rows of `stride`), counts,
+// statuses, and `extra` more bytes of the caller's. Up to kStaged bytes go
+// through pinned memory (a copy to pageable memory costs about 10 us however
+// small it is: 1 query's four arrays took 40 of 183 us); larger ones, where
+// the bytes decide, go to the caller's arrays directly.
+struct Outputs {
+    static constexpr size_t kStaged = size_t(1) << 20;
+    DBuf dev;
+    void* host = nullptr;
+    size_t host_bytes = 0, rows = 0, stride = 0, tail = 0;
+    uint64_t* keys() const { return dev.as<uint64_t>(); }
+    float* dist() const { return reinterpret_cast<float*>(keys() + rows * stride); }
+    uint32_t* count() const { return reinterpret_cast<uint32_t*>(dist() + rows * stride); }
+    int32_t* status() const { return reinterpret_cast<int32_t*>(count() + rows); }
+    uint32_t* extra() const { return reinterpret_cast<uint32_t*>(status() + rows); }
+    size_t bytes() const { return rows * stride * 12 + rows * 8 + tail; }
+    cudaError_t ensure(size_t nq, size_t row_stride, size_t extra_bytes = 0) {
+        rows = nq;
+        stride = row_stride;
+        tail = extra_bytes;
+        return dev.ensure(std::max<size_t>(bytes(), 16));
+    }
+    // Enqueues the copies, waits for the stream, and fills the caller's arrays
+    // (`extra_out` with the extra bytes; `rows_out` false: no keys and distances).
+    cudaError_t fetch(cudaStream_t st, uint64_t* k, float* d, uint32_t* c, int32_t* s, bool rows_out = true,
+                      void* extra_out = nullptr) {
+        const size_t kb = rows_out ? rows * stride * 8 : 0, db = rows_out ? rows * stride * 4 : 0;
+        if (bytes() <= kStaged) {
+            if (host_bytes < bytes()) {
+                if (host) cudaFreeHost(host);
+                host = nullptr;
+                host_bytes = 0;
+                size_t want = 16384;
+                while (want < bytes()) want <<= 1;
+                if (cudaHostAlloc(&host, want, cudaHostAllocDefault) == cudaSuccess) host_bytes = want;
+                else cudaGetLastError();  // no pinned memory: copy directly
+            }
+            if (host_bytes >= bytes()) {
+                cudaError_t e = cudaMemcpyAsync(host, dev.p, bytes(), cudaMemcpyDeviceToHost, st);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                if (e != cudaSuccess) return e;
+                const char* h = static_cast<const char*>(host);
+                auto at = [&](const void* p) { return h + (static_cast<const char*>(p) - static_cast<const char*>(dev.p)); };
+                if (kb) std::memcpy(k, at(keys()), kb);
+                if (db) std::memcpy(d, at(dist()), db);
+                std::memcpy(c, at(count()), rows * 4);
+                std::memcpy(s, at(status()), rows * 4);
+                if (extra_out) std::memcpy(extra_out, at(extra()), tail);
+                return cudaSuccess;
+            }
+        }
+        cudaError_t e = cudaSuccess;
+        auto copy = [&](void* to, const void* from, size_t n) {
+            if (e == cudaSuccess && n) e = cudaMemcpyAsync(to, from, n, cudaMemcpyDeviceToHost, st);
+        };
+        copy(c, count(), rows * 4);
+        copy(s, status(), rows * 4);
+        copy(k, keys(), kb);
+        copy(d, dist(), db);
+        if (extra_out) copy(extra_out, extra(), tail);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    }
+    void release() {
+        dev.release();
+        if (host) cudaFreeHost(host);
+        host = nullptr;
+        host_bytes = 0;
+    }
+};
+
 // One concurrent call's stream and scratch.
 struct Slot {
     cudaStream_t stream = nullptr;
-    DBuf q, ks, efs, fbits, fused, fids, okeys, odist, ocount, ostatus, work, overflow, counters;
+    DBuf q, ks, efs, fbits, fused, fids, work, overflow, counters;
+    hnswgpu::Outputs out;
     DBuf g_results, g_cands, g_visited;
     uint32_t g_warps = 0, g_ef_cap = 0, g_cand_cap = 0;
     uint64_t g_words = 0;
@@ -87,10 +161,11 @@ struct Slot {
     DBuf team_bits, team_far, order;      // team traversal: visited bitmaps, far candidates, query order
     size_t last_nq = 0;
     ~Slot() {
-        for (DBuf* b : {&q, &ks, &efs, &fbits, &fused, &fids, &okeys, &odist, &ocount, &ostatus, &work, &overflow, &counters,
+        for (DBuf* b : {&q, &ks, &efs, &fbits, &fused, &fids, &work, &overflow, &counters,
                         &g_results, &g_cands, &g_visited, &spill_bits, &spill_cands, &cold_pool, &cold_tab, &last_pool,
                         &last_tab, &overflow2, &planned, &team_bits, &team_far, &order})
             b->release();
+        out.release();
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -187,6 +262,10 @@ struct hnsw_gpu_index {
     };
     std::mutex tune_mu;
     Tuned tuned[33];
+    // The occupancy heuristic's choices (pick_geometry, about twenty occupancy
+    // queries) by ef capacity, mode, filter and visited-tag setting.
+    std::mutex plan_mu;
+    std::map<uint64_t, hnswgpu::SearchGeometry> plans;
     cudaEvent_t dev_done = nullptr;
     // Tensor-core traversal rows, built on first use (tc_mu): BF16 high
     // parts, low parts (BF16X3), f32 squared norms (L2).
@@ -218,12 +297,13 @@ struct hnsw_gpu_brute {
     DBuf krank, skeys;  // key ranks and sorted keys, when the keys do not ascend
     SlotPool slots;
     std::mutex mu;
-    DBuf qprep, part, minima, okeys, odist, ocount, ostatus, q;
+    DBuf qprep, part, minima, q;
+    hnswgpu::Outputs out;
     DBuf fbits, fused, fids;  // filter bitmaps, flags and bitmap ids of a filtered search
     // Tensor-core path: BF16 operand rows per term count (index 0: 1 term, 1: 3 terms).
     DBuf bop[2], xnorm2;
     uint32_t bop_kp[2] = {0, 0};
-    DBuf aop, dense, thr1, thr2, margin, qnorm2, ccount, cand, err;
+    DBuf aop, dense, thr1, thr2, margin, qnorm2, cand;
     uint64_t last_candidates = 0, last_queries = 0;
     float last_ms[4] = {0, 0, 0, 0};
     long long wait_budget = 4000000000ll;  // tensor-core pipeline waits, clock cycles
@@ -233,10 +313,11 @@ struct hnsw_gpu_brute {
     cudaStream_t stream = nullptr;
     ~hnsw_gpu_brute() {
         DeviceGuard g(device);
-        for (DBuf* b : {&base, &keys, &krank, &skeys, &qprep, &part, &minima, &okeys, &odist, &ocount, &ostatus, &q, &fbits, &fused, &fids,
+        for (DBuf* b : {&base, &keys, &krank, &skeys, &qprep, &part, &minima, &q, &fbits, &fused, &fids,
                         &bop[0], &bop[1], &xnorm2,
-                        &aop, &dense, &thr1, &thr2, &margin, &qnorm2, &ccount, &cand, &err})
+                        &aop, &dense, &thr1, &thr2, &margin, &qnorm2, &cand})
             b->release();
+        out.release();
         for (cudaEvent_t& e : ev)
             if (e) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
