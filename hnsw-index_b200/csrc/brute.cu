@@ -565,69 +565,98 @@ __global__ void brute_merge_kernel(BruteArgs a, uint32_t kk, uint32_t nslices) {
     if (lane == 0) a.out_count[q] = want;
 }
 
-// Exact re-rank of tensor-core candidates (one warp per query): every
-// candidate whose approximate distance is <= thr2[q] gets its FP32 distance
-// in the reference kernel order; a top-k list ordered by (total_cmp distance,
-// key) keeps the best (src/brute.rs:131-160). A query whose candidate list
-// overflowed gets status 25 and is re-run by the exact FP32 kernels.
-__global__ void brute_rerank_kernel(BruteArgs a, const uint64_t* __restrict__ cand,
-                                    const uint32_t* __restrict__ cand_count, uint32_t cand_cap,
-                                    const float* __restrict__ thr2, uint32_t kk) {
+// Exact re-rank of tensor-core candidates: every candidate whose approximate
+// distance is <= thr2[q] gets its FP32 distance in the reference kernel order;
+// a top-k list ordered by (total_cmp distance, key) keeps the best
+// (src/brute.rs:131-160). A query whose candidate list overflowed gets status
+// 25 and is re-run by the exact FP32 kernels. A block per query: the rows that
+// pass are collected 1024 candidates at a time, each warp scores eight of them
+// per memory round trip and keeps a list of its own, and warp 0 merges the
+// lists. (One warp per query took 346 us for 2000 queries of 768 dimensions
+// with 1,250 candidates each, waiting on its row loads 22 of 27 cycles.)
+// SMEM_Q: the query in shared memory (left in global memory when it is large).
+constexpr uint32_t kRerankBatch = 1024;
+template <bool SMEM_Q>
+__global__ void __launch_bounds__(256) brute_rerank_kernel(BruteArgs a, const uint64_t* __restrict__ cand,
+                                                           const uint32_t* __restrict__ cand_count, uint32_t cand_cap,
+                                                           const float* __restrict__ thr2, uint32_t kk) {
     extern __shared__ __align__(16) char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t q = blockIdx.x * (blockDim.x >> 5) + uint32_t(warp);
-    const uint32_t nw = blockDim.x >> 5;
-    uint64_t* lists = reinterpret_cast<uint64_t*>(smem);
-    uint64_t* bufs = lists + size_t(nw) * kk;
-    uint32_t* pos = reinterpret_cast<uint32_t*>(bufs + size_t(nw) * 32) + warp * 32;
-    if (q >= a.nq) return;
+    __shared__ uint32_t rows[kRerankBatch];
+    __shared__ uint32_t nrows, sizes[8];
+    const uint32_t q = blockIdx.x, nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     if (a.out_status[q] != 0) {
-        if (lane == 0) a.out_count[q] = 0;
+        if (threadIdx.x == 0) a.out_count[q] = 0;
         return;
     }
     const uint32_t total = cand_count[q];
     if (total > cand_cap) {
-        if (lane == 0) a.out_status[q] = 25;
+        if (threadIdx.x == 0) a.out_status[q] = 25;
         return;
     }
-    const float t2 = thr2[q];
+    float* sq = reinterpret_cast<float*>(smem);
+    uint64_t* lists = reinterpret_cast<uint64_t*>(sq + (SMEM_Q ? a.dp : 0));
+    uint64_t* bufs = lists + size_t(nw) * kk;
     const float* qv = a.qprep + size_t(q) * a.dp;
+    if (SMEM_Q) {
+        for (uint32_t i = threadIdx.x * 4; i < a.dp; i += blockDim.x * 4)
+            *reinterpret_cast<float4*>(sq + i) = *reinterpret_cast<const float4*>(qv + i);
+        qv = sq;
+    }
+    const float t2 = thr2[q];
     const uint64_t* C = cand + size_t(q) * cand_cap;
     const int g = lane >> 3, g8 = lane & 7;
     TopList t{lists + size_t(warp) * kk, bufs + warp * 32, 0, 0};
-    for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t i = base + uint32_t(lane);
-        uint32_t row = 0;
-        bool pass = false;
-        if (i < total) {
+    for (uint32_t base = 0; base < total; base += kRerankBatch) {
+        __syncthreads();
+        if (threadIdx.x == 0) nrows = 0;
+        __syncthreads();
+        for (uint32_t i = base + threadIdx.x; i < min(total, base + kRerankBatch); i += blockDim.x) {
             const uint64_t c = C[i];
-            pass = __uint_as_float(uint32_t(c >> 32)) <= t2;
-            row = uint32_t(c);
+            if (__uint_as_float(uint32_t(c >> 32)) <= t2) rows[atomicAdd(&nrows, 1u)] = uint32_t(c);
         }
-        const uint32_t P = __ballot_sync(kFull, pass);
-        if (pass) pos[__popc(P & ((1u << lane) - 1u))] = row;
-        __syncwarp();
-        const uint32_t np = __popc(P);
-        for (uint32_t r = 0; r < np; r += 4) {
-            const uint32_t slot = r + uint32_t(g);
-            const uint32_t rrow = pos[slot < np ? slot : 0];
-            const float* xr = a.base + size_t(rrow) * a.dp;
-            float sum = a.metric == 0 ? group_sum<true>(xr, qv, int(a.dim), g8) : group_sum<false>(xr, qv, int(a.dim), g8);
-            const float d = metric_from_sum(a.metric, sum);
-            const uint64_t e = brute_entry(a, d, rrow);
-            const uint64_t worst = t.n == kk ? t.L[kk - 1] : ~0ull;
-            const uint32_t W = __ballot_sync(kFull, g8 == 0 && slot < np && e < worst);
-            if (W) top_push(t, W, e, kk);
+        __syncthreads();
+        const uint32_t np = nrows;
+        for (uint32_t r = warp * 8; r < np; r += nw * 8) {
+            const uint32_t sa = r + uint32_t(g), sb = sa + 4;
+            const uint32_t ra = rows[min(sa, np - 1)], rb = rows[min(sb, np - 1)];
+            const float* xa = a.base + size_t(ra) * a.dp;
+            const float* xb = a.base + size_t(rb) * a.dp;
+            float d0, d1;
+            if (a.metric == 0) group_sum2<true>(xa, xb, qv, int(a.dim), g8, d0, d1);
+            else group_sum2<false>(xa, xb, qv, int(a.dim), g8, d0, d1);
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const bool in = g8 == 0 && (h ? sb : sa) < np;
+                const uint64_t e = in ? brute_entry(a, metric_from_sum(a.metric, h ? d1 : d0), h ? rb : ra) : ~0ull;
+                const uint64_t worst = t.n == kk ? t.L[kk - 1] : ~0ull;
+                const uint32_t W = __ballot_sync(kFull, e < worst);
+                if (W) top_push(t, W, e, kk);
+            }
         }
-        __syncwarp();
     }
     if (t.cnt) top_flush(t, kk);
-    const uint32_t want = min(a.k, a.n);
-    for (uint32_t i = lane; i < t.n && i < want; i += 32) {
+    if (lane == 0) sizes[warp] = t.n;
+    __syncthreads();
+    if (warp != 0) return;
+    for (uint32_t w2 = 1; w2 < nw; ++w2) {
+        const uint64_t* other = lists + size_t(w2) * kk;
+        const uint32_t n2 = sizes[w2];
+        for (uint32_t b = 0; b < n2; b += 32) {
+            const uint64_t x = b + uint32_t(lane) < n2 ? other[b + lane] : ~0ull;
+            const uint32_t S = __ballot_sync(kFull, x < (t.n == kk ? t.L[kk - 1] : ~0ull));
+            if (S == 0) break;
+            batch_merge_gather(t.L, 0, t.n, S, x, kk, t.B);
+            __syncwarp();
+            t.n = min(t.n + uint32_t(__popc(S)), kk);
+        }
+    }
+    const uint32_t want = min(t.n, min(a.k, a.n));
+    for (uint32_t i = lane; i < want; i += 32) {
         a.out_keys[size_t(q) * a.k + i] = __ldg(a.skeys + uint32_t(t.L[i]));
         a.out_dist[size_t(q) * a.k + i] = kdec(uint32_t(t.L[i] >> 32));
     }
-    if (lane == 0) a.out_count[q] = min(t.n, want);
+    if (lane == 0) a.out_count[q] = want;
 }
 
 }  // namespace dev
@@ -640,11 +669,14 @@ cudaError_t launch_brute_prep(const BruteArgs& a, cudaStream_t stream) {
 cudaError_t launch_brute_rerank(const BruteArgs& a, const uint64_t* cand, const uint32_t* cand_count, uint32_t cand_cap,
                                 const float* thr2, cudaStream_t stream) {
     const uint32_t kk = std::max<uint32_t>(1, std::min<uint32_t>(a.k, a.n ? a.n : 1));
-    const uint32_t wpb = 4;
-    const size_t smem = size_t(wpb) * (kk + 32) * 8 + size_t(wpb) * 32 * 4;
-    cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(dev::brute_rerank_kernel));
+    // Warps per query: eight while the queries do not fill the SMs.
+    const uint32_t nw = a.nq >= 1024 ? 4 : 8;
+    const bool smem_q = a.dp <= 16384;
+    const size_t smem = (smem_q ? size_t(a.dp) * 4 : 0) + size_t(nw) * (kk + 32) * 8;
+    auto kern = smem_q ? dev::brute_rerank_kernel<true> : dev::brute_rerank_kernel<false>;
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kern));
     if (e != cudaSuccess) return e;
-    dev::brute_rerank_kernel<<<(a.nq + wpb - 1) / wpb, 32 * wpb, smem, stream>>>(a, cand, cand_count, cand_cap, thr2, kk);
+    kern<<<a.nq, 32 * nw, smem, stream>>>(a, cand, cand_count, cand_cap, thr2, kk);
     return cudaGetLastError();
 }
 

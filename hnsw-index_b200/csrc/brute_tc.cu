@@ -191,22 +191,46 @@ __device__ __forceinline__ float tile_distance(const TcScoreArgs& a, float s, fl
 struct EpiConsts {
     int metric;
     uint32_t n;
-    const float* xnorm2;
+    const float* xn;  // shared memory: the squared norms of the tile's 256 rows (L2)
 };
-__device__ __forceinline__ float row_distance(const EpiConsts& e, float s, float qn, uint32_t row) {
-    if (e.metric == 0) return qn + (row < e.n ? __ldg(e.xnorm2 + row) : 0.0f) - 2.0f * s;
+__device__ __forceinline__ float row_distance(const EpiConsts& e, float s, float qn, float xn) {
+    if (e.metric == 0) return qn + xn - 2.0f * s;
     if (e.metric == 1) return -s;
     return 1.0f - s;
 }
+
+// The squared norms of a tile's rows for the L2 epilogues, lane l holding
+// those of rows 4l.. and 128 + 4l..: loaded while the MMAs run and put into
+// the epilogue warp's shared memory when its previous tile is done. (Read
+// per element from global memory they were what bounded an L2 tile: 300
+// queries x 100k x 200 in BF16 took 57 us for the sample and 90 us for the
+// candidate pass.)
+struct TileNorms {
+    float4 a, b;
+    __device__ __forceinline__ void load(const TcScoreArgs& args, uint32_t row_base) {
+        if (args.metric != 0) return;
+        const float4* x = reinterpret_cast<const float4*>(args.xnorm2 + row_base) + (threadIdx.x & 31);
+        a = __ldg(x);
+        b = __ldg(x + 32);
+    }
+    __device__ __forceinline__ void store(const TcScoreArgs& args, float* xn) const {
+        if (args.metric != 0) return;
+        __syncwarp();
+        reinterpret_cast<float4*>(xn)[threadIdx.x & 31] = a;
+        reinterpret_cast<float4*>(xn)[32 + (threadIdx.x & 31)] = b;
+        __syncwarp();
+    }
+};
 
 // Dense epilogue (threshold sample pass): this lane's query q against the
 // 256 rows row_base .. row_base + 255 held in TMEM columns taddr .. taddr +
 // 255 of its lane; every distance of the sample's row range is written,
 // four at a time (+inf past the last row). All 32 lanes call.
-__device__ __forceinline__ void epilogue_dense(const TcScoreArgs& a, uint32_t taddr, uint32_t q, uint32_t row_base) {
+__device__ __forceinline__ void epilogue_dense(const TcScoreArgs& a, uint32_t taddr, uint32_t q, uint32_t row_base,
+                                               const float* xn) {
     const bool qvalid = q < a.nq;
     const float qn = (qvalid && a.qnorm2) ? a.qnorm2[q] : 0.0f;
-    const EpiConsts e{a.metric, a.n, a.xnorm2};
+    const EpiConsts e{a.metric, a.n, xn};
     for (uint32_t c = 0; c < kTileN / 32; ++c) {
         uint32_t v[32];
         __syncwarp();
@@ -219,10 +243,13 @@ __device__ __forceinline__ void epilogue_dense(const TcScoreArgs& a, uint32_t ta
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
             float d[4];
+            const float4 x4 = e.metric == 0 ? reinterpret_cast<const float4*>(e.xn)[c * 8 + j / 4]
+                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float xs[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const uint32_t row = row0 + uint32_t(j + i);
-                d[i] = row < e.n ? row_distance(e, __uint_as_float(v[j + i]), qn, row) : __int_as_float(0x7f800000);
+                d[i] = row < e.n ? row_distance(e, __uint_as_float(v[j + i]), qn, xs[i]) : __int_as_float(0x7f800000);
             }
             out[j / 4] = make_float4(d[0], d[1], d[2], d[3]);
         }
@@ -235,10 +262,11 @@ __device__ __forceinline__ void epilogue_dense(const TcScoreArgs& a, uint32_t ta
 // consecutive words). A chunk of 32 columns adds at most 32, so a warp
 // appends its staged entries before a chunk whenever a lane holds more than
 // kStageDepth - 32.
-constexpr uint32_t kStageDepth = 48;
+constexpr uint32_t kStageDepth = 44;
 // One more row per lane takes the stores of entries that do not pass, so the
 // scan has no branch per element.
-constexpr uint32_t kStageBytesPerWarp = (kStageDepth + 1) * 32 * 5;  // 7.7 KB
+constexpr uint32_t kNormBytes = kTileN * 4;                           // TileNorms of the warp
+constexpr uint32_t kStageBytesPerWarp = kNormBytes + (kStageDepth + 1) * 32 * 5;  // 8.2 KB
 
 // Appends this lane's n staged entries to its query's candidates (one
 // reservation).
@@ -259,17 +287,18 @@ __device__ __forceinline__ void flush_stage(const TcScoreArgs& a, const float* s
 // kStageDepth, and only a passing one advances n. `lim` is the number of
 // valid columns (0 for a padding query). METRIC as in tile_distance.
 template <int METRIC>
-__device__ __forceinline__ void stage_chunk_m(const EpiConsts& e, const uint32_t (&v)[32], uint32_t row_base,
+__device__ __forceinline__ void stage_chunk_m(const EpiConsts& e, const uint32_t (&v)[32],
                                               uint32_t col0, uint32_t lim, float thr, float qn, float* sd,
                                               uint8_t* sr, uint32_t& n) {
     const uint32_t lane = threadIdx.x & 31;
+    float4 x4;
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
         const float s = __uint_as_float(v[j]);
         float dist;
         if (METRIC == 0) {
-            const uint32_t row = row_base + col0 + uint32_t(j);
-            dist = qn + (row < e.n ? __ldg(e.xnorm2 + row) : 0.0f) - 2.0f * s;
+            if (j % 4 == 0) x4 = reinterpret_cast<const float4*>(e.xn)[(col0 + uint32_t(j)) / 4];
+            dist = qn + (j % 4 == 0 ? x4.x : (j % 4 == 1 ? x4.y : (j % 4 == 2 ? x4.z : x4.w))) - 2.0f * s;
         } else if (METRIC == 1) {
             dist = -s;
         } else {
@@ -282,12 +311,12 @@ __device__ __forceinline__ void stage_chunk_m(const EpiConsts& e, const uint32_t
         n += pass ? 1u : 0u;
     }
 }
-__device__ __forceinline__ void stage_chunk(const EpiConsts& e, const uint32_t (&v)[32], uint32_t row_base,
+__device__ __forceinline__ void stage_chunk(const EpiConsts& e, const uint32_t (&v)[32],
                                             uint32_t col0, uint32_t lim, float thr, float qn, float* sd, uint8_t* sr,
                                             uint32_t& n) {
-    if (e.metric == 0) stage_chunk_m<0>(e, v, row_base, col0, lim, thr, qn, sd, sr, n);
-    else if (e.metric == 1) stage_chunk_m<1>(e, v, row_base, col0, lim, thr, qn, sd, sr, n);
-    else stage_chunk_m<2>(e, v, row_base, col0, lim, thr, qn, sd, sr, n);
+    if (e.metric == 0) stage_chunk_m<0>(e, v, col0, lim, thr, qn, sd, sr, n);
+    else if (e.metric == 1) stage_chunk_m<1>(e, v, col0, lim, thr, qn, sd, sr, n);
+    else stage_chunk_m<2>(e, v, col0, lim, thr, qn, sd, sr, n);
 }
 
 // Candidate mode, one pass: the accumulator's eight 32-column chunks are
@@ -298,9 +327,9 @@ template <typename Release>
 __device__ __forceinline__ void epilogue_candidates(const TcScoreArgs& a, uint32_t taddr, uint32_t q,
                                                     uint32_t row_base, float thr, float qn, unsigned char* stage,
                                                     Release release) {
-    const EpiConsts e{a.metric, a.n, a.xnorm2};
-    float* sd = reinterpret_cast<float*>(stage);
-    uint8_t* sr = stage + (kStageDepth + 1) * 32 * 4;
+    const EpiConsts e{a.metric, a.n, reinterpret_cast<const float*>(stage)};
+    float* sd = reinterpret_cast<float*>(stage + kNormBytes);
+    uint8_t* sr = stage + kNormBytes + (kStageDepth + 1) * 32 * 4;
     // Valid columns of this tile for this lane's query.
     const uint32_t valid = q < a.nq ? (row_base < e.n ? min(e.n - row_base, kTileN) : 0u) : 0u;
     uint32_t n = 0;
@@ -315,7 +344,7 @@ __device__ __forceinline__ void epilogue_candidates(const TcScoreArgs& a, uint32
             n = 0;
         }
         __syncwarp();
-        stage_chunk(e, va, row_base, c * 32, valid > c * 32 ? min(valid - c * 32, 32u) : 0u, thr, qn, sd, sr, n);
+        stage_chunk(e, va, c * 32, valid > c * 32 ? min(valid - c * 32, 32u) : 0u, thr, qn, sd, sr, n);
         __syncwarp();
         tmem_wait_regs(vb);
         if (c + 2 < kTileN / 32) tmem_ld32_async(taddr + (c + 2) * 32, va);
@@ -325,7 +354,7 @@ __device__ __forceinline__ void epilogue_candidates(const TcScoreArgs& a, uint32
             n = 0;
         }
         __syncwarp();
-        stage_chunk(e, vb, row_base, (c + 1) * 32, valid > (c + 1) * 32 ? min(valid - (c + 1) * 32, 32u) : 0u, thr,
+        stage_chunk(e, vb, (c + 1) * 32, valid > (c + 1) * 32 ? min(valid - (c + 1) * 32, 32u) : 0u, thr,
                     qn, sd, sr, n);
         __syncwarp();
         if (c + 2 < kTileN / 32) tmem_wait_regs(va);
@@ -475,8 +504,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             // The query's threshold and norm load while the MMAs run.
             const float thr = (q < a.nq && a.thr) ? a.thr[q] : 0.0f;
             const float qn = (q < a.nq && a.qnorm2) ? a.qnorm2[q] : 0.0f;
+            TileNorms norms;
+            norms.load(a, nt * kTileN);
             const bool got = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[b], use & 1u, a.err, a.wait_budget));
             if (!got) break;
+            norms.store(a, reinterpret_cast<float*>(stage));
             tc_fence_after();
             const uint32_t taddr = tmem_base + (lane_base << 16) + b * kTileN;
             auto release = [&]() {
@@ -485,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (lane == 0) mbar_arrive(&acc_empty[b]);
             };
             if (a.dense) {
-                epilogue_dense(a, taddr, q, nt * kTileN);
+                epilogue_dense(a, taddr, q, nt * kTileN, reinterpret_cast<const float*>(stage));
                 release();
             } else {
                 epilogue_candidates(a, taddr, q, nt * kTileN, thr, qn, stage, release);
@@ -746,8 +778,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const uint32_t q = (2 * qp2 + rank) * kTileM + lane_base + uint32_t(lane);
             const float thr = (q < a.nq && a.thr) ? a.thr[q] : 0.0f;
             const float qn = (q < a.nq && a.qnorm2) ? a.qnorm2[q] : 0.0f;
+            TileNorms norms;
+            norms.load(a, nt * kTileN);
             const bool got = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[b], use & 1u, a.err, a.wait_budget));
             if (!got) break;
+            norms.store(a, reinterpret_cast<float*>(stage));
             tc_fence_after();
             const uint32_t taddr = tmem_base + (lane_base << 16) + b * kTileN;
             auto release = [&]() {
@@ -759,7 +794,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
             };
             if (a.dense) {
-                epilogue_dense(a, taddr, q, nt * kTileN);
+                epilogue_dense(a, taddr, q, nt * kTileN, reinterpret_cast<const float*>(stage));
                 release();
             } else {
                 epilogue_candidates(a, taddr, q, nt * kTileN, thr, qn, stage, release);
@@ -811,18 +846,23 @@ __global__ void row_norms_kernel(const float* __restrict__ src, uint32_t n, uint
 }
 
 // k-th smallest value of each query's row of `vals` (count entries, +inf
-// padding allowed) by a 4-pass radix select on the order-preserving key; the
-// threshold written is that value + margin[q] (or +inf when count < k).
-__global__ void kth_threshold_kernel(const float* __restrict__ vals, uint32_t ld, const uint32_t* __restrict__ counts,
-                                     const uint64_t* __restrict__ packed, uint32_t packed_cap, uint32_t nq, uint32_t k,
-                                     const float* __restrict__ margin, float* __restrict__ thr_out) {
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t s_prefix, s_rank;
-    const uint32_t q = blockIdx.x;
-    if (q >= nq) return;
+// padding allowed); the threshold written is that value + margin[q] (or +inf
+// when count < k). A block per query: the order-preserving keys are held in
+// registers when there are up to 16,384 of them, and a radix selection narrows
+// the window [smallest, largest] by 1024 bins a pass (fixed byte digits put
+// most keys of a sample into one bin, re-read them four times and scanned the
+// bins with one thread: 185 us for 2000 queries' samples of 16,384, 41 us for
+// their 1,250 candidates).
+constexpr uint32_t kKthThreads = 512, kKthCache = 32, kKthBins = 1024;
+__global__ void __launch_bounds__(kKthThreads)
+    kth_threshold_kernel(const float* __restrict__ vals, uint32_t ld, const uint32_t* __restrict__ counts,
+                         const uint64_t* __restrict__ packed, uint32_t packed_cap, uint32_t nq, uint32_t k,
+                         const float* __restrict__ margin, float* __restrict__ thr_out) {
+    __shared__ uint32_t hist[kKthBins + kKthBins / 32], wmin[kKthThreads / 32], wmax[kKthThreads / 32], s_bin, s_below;
+    const uint32_t q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t n = counts ? min(counts[q], packed_cap) : ld;
     if (n < k || k == 0) {
-        if (threadIdx.x == 0) thr_out[q] = __int_as_float(0x7f800000);
+        if (tid == 0) thr_out[q] = __int_as_float(0x7f800000);
         return;
     }
     auto key_at = [&](uint32_t i) -> uint32_t {
@@ -830,32 +870,94 @@ __global__ void kth_threshold_kernel(const float* __restrict__ vals, uint32_t ld
                                : vals[size_t(q) * ld + i];
         return dev::fkey(v);
     };
-    uint32_t prefix = 0, rank = k;  // find the rank-th smallest key (1-based)
-    for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 24 - 8 * pass;
-        for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-        __syncthreads();
-        const uint32_t mask_hi = pass == 0 ? 0u : (0xFFFFFFFFu << (32 - 8 * pass));
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t key = key_at(i);
-            if ((key & mask_hi) == (prefix & mask_hi)) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t acc = 0, digit = 0;
-            for (; digit < 256; ++digit) {
-                if (acc + hist[digit] >= rank) break;
-                acc += hist[digit];
+    // A word of padding per 32 bins: the scan's lanes read 32 bins each.
+    auto bin_at = [](uint32_t b) { return b + (b >> 5); };
+    const bool cached = n <= kKthThreads * kKthCache;
+    uint32_t keys[kKthCache];
+    uint32_t mn = 0xFFFFFFFFu, mx = 0;
+    if (cached) {
+#pragma unroll
+        for (uint32_t g = 0; g < kKthCache; g += 8)
+            if (g * kKthThreads < n) {
+#pragma unroll
+                for (uint32_t j = g; j < g + 8; ++j) {
+                    const uint32_t i = tid + j * kKthThreads;
+                    keys[j] = i < n ? key_at(i) : 0u;
+                }
+#pragma unroll
+                for (uint32_t j = g; j < g + 8; ++j)
+                    if (tid + j * kKthThreads < n) {
+                        mn = min(mn, keys[j]);
+                        mx = max(mx, keys[j]);
+                    }
             }
-            s_prefix = prefix | (digit << shift);
-            s_rank = rank - acc;
+    } else {
+        for (uint32_t i = tid; i < n; i += kKthThreads) {
+            const uint32_t key = key_at(i);
+            mn = min(mn, key);
+            mx = max(mx, key);
+        }
+    }
+    mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    if (lane == 0) {
+        wmin[warp] = mn;
+        wmax[warp] = mx;
+    }
+    __syncthreads();
+    for (uint32_t i = 0; i < kKthThreads / 32; ++i) {
+        mn = min(mn, wmin[i]);
+        mx = max(mx, wmax[i]);
+    }
+    // The rank-th smallest key (1-based) of those in [lo, lo + 2^bits).
+    uint32_t lo = mn, rank = k;
+    int bits = 32 - __clz(int(mx - mn));
+    while (bits > 0) {
+        const int sh = max(bits - 10, 0);
+        for (uint32_t i = tid; i < kKthBins + kKthBins / 32; i += kKthThreads) hist[i] = 0;
+        __syncthreads();
+        auto count = [&](uint32_t key) {
+            const uint32_t off = key - lo;
+            if (key >= lo && (bits >= 32 || (off >> bits) == 0)) atomicAdd(&hist[bin_at(off >> sh)], 1u);
+        };
+        if (cached) {
+#pragma unroll
+            for (uint32_t g = 0; g < kKthCache; g += 8)
+                if (g * kKthThreads < n) {
+#pragma unroll
+                    for (uint32_t j = g; j < g + 8; ++j)
+                        if (tid + j * kKthThreads < n) count(keys[j]);
+                }
+        } else {
+            for (uint32_t i = tid; i < n; i += kKthThreads) count(key_at(i));
         }
         __syncthreads();
-        prefix = s_prefix;
-        rank = s_rank;
+        if (warp == 0) {
+            constexpr uint32_t P = kKthBins / 32;
+            uint32_t sum = 0;
+            static_assert(P == 32, "one padding word per lane's bins");
+#pragma unroll 8
+            for (uint32_t i = 0; i < P; ++i) sum += hist[bin_at(lane * P + i)];
+            uint32_t incl = sum;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                if (lane >= uint32_t(off)) incl += o;
+            }
+            if (incl >= rank && incl - sum < rank) {  // one lane: its bins hold the key
+                uint32_t below = incl - sum, bin = lane * P;
+                while (below + hist[bin_at(bin)] < rank) below += hist[bin_at(bin++)];
+                s_bin = bin;
+                s_below = below;
+            }
+        }
+        __syncthreads();
+        rank -= s_below;
+        lo += s_bin << sh;
+        bits = sh;
         __syncthreads();
     }
-    if (threadIdx.x == 0) thr_out[q] = dev::kdec(prefix) + margin[q];
+    if (tid == 0) thr_out[q] = dev::kdec(lo) + margin[q];
 }
 
 // Per-query error margin 2E in distance units (see tc_margins).
@@ -973,7 +1075,7 @@ cudaError_t tc_kth_threshold(const float* vals, uint32_t ld, const uint32_t* cou
                              uint32_t packed_cap, uint32_t nq, uint32_t k, const float* margin, float* thr_out,
                              cudaStream_t stream) {
     if (nq == 0) return cudaSuccess;
-    tc::kth_threshold_kernel<<<nq, 256, 0, stream>>>(vals, ld, counts, packed, packed_cap, nq, k, margin, thr_out);
+    tc::kth_threshold_kernel<<<nq, tc::kKthThreads, 0, stream>>>(vals, ld, counts, packed, packed_cap, nq, k, margin, thr_out);
     return cudaGetLastError();
 }
 
