@@ -134,8 +134,7 @@ SearchGeometry pick_geometry(uint32_t ef_max, uint32_t dp, uint32_t dc, bool per
 }  // namespace hnswgpu
 
 // Ensures the retry workspaces of a slot (visited bitmap over all nodes, heaps).
-static int ensure_retry(hnsw_gpu_index* gi, Slot* s, uint32_t ef_cap) {
-    const uint32_t warps = uint32_t(gi->num_sms) * 4;
+static int ensure_retry(hnsw_gpu_index* gi, Slot* s, uint32_t ef_cap, uint32_t warps) {
     const uint32_t cand_cap = std::max<uint32_t>(1u << 14, 4 * ef_cap);
     const uint64_t words = (uint64_t(gi->view.n) + 31) / 32 + 1;
     CU(s->g_results.ensure(size_t(warps) * (ef_cap + 1) * 8), "cudaMalloc retry results");
@@ -237,13 +236,12 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     }
     if (!persistent) geo.cold = 0;  // cold lists need the persistent warps' chunk tables
     // work: [0] next query, [1] overflow count, [2] [3] cold chunks handed
-    // out by the fast (cold variant) and retry kernels, [4] last-resort count.
+    // out by the fast (cold variant) and retry kernels, [4] last-resort count,
+    // [5] route, [6] next query of the teams' retry pass.
     CU(s->work.ensure(32), "cudaMalloc work counters");
     CU(s->overflow.ensure(std::max<size_t>(nq, 1) * 4), "cudaMalloc overflow list");
     CU(s->overflow2.ensure(std::max<size_t>(nq, 1) * 4), "cudaMalloc overflow list");
     CU(cudaMemsetAsync(s->work.p, 0, 32, stream), "memset work counters");
-    int r = ensure_retry(gi, s, std::max(geo.ef_cap, round_up(ef_max, 32)));
-    if (r != HNSW_OK) return r;
     SearchArgs a;
     a.ix = gi->view;
     a.queries = d_q;
@@ -296,17 +294,32 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
     if (heuristic && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
-    if (team.blocks) {
-        // Without memory for the teams the batch takes the warp kernels.
-        const size_t row = team.bitmap_words ? 0 : ((size_t(gi->view.n) + 31) / 32 + 3) / 4 * 16;
-        cudaError_t e = s->team_far.ensure(size_t(team.blocks) * team.far_cap * 8);
-        if (e == cudaSuccess && row) e = s->team_bits.ensure(size_t(team.blocks) * row);
+    // Without memory for the teams the batch takes the warp kernels.
+    const uint32_t bit_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
+    auto ensure_team = [&](TeamGeometry& g) {
+        if (!g.blocks) return;
+        cudaError_t e = s->team_far.ensure(size_t(g.blocks) * g.far_cap * 8);
+        if (e == cudaSuccess && !g.bitmap_words) e = s->team_bits.ensure(size_t(g.blocks) * bit_words * 4);
         if (e != cudaSuccess) {
             cudaGetLastError();
-            team = TeamGeometry();
+            g = TeamGeometry();
         }
-    }
+    };
+    ensure_team(team);
     const bool warp_route = !team.blocks || !small;
+    // Queries that outgrow a warp's scratch are redone by teams (one per SM):
+    // a warp of the retry kernel takes milliseconds for one, and the batch
+    // waits for it.
+    TeamGeometry redo;
+    if (heuristic && !o.traversal && tags == 0 && warp_route && ef_max <= 1024) {
+        SearchArgs one = a;
+        one.nq = uint32_t(gi->num_sms);
+        CU(plan_search_team(one, ef_max, gi->num_sms, &redo), "team occupancy");
+        ensure_team(redo);
+    }
+    int r = ensure_retry(gi, s, std::max(geo.ef_cap, round_up(ef_max, 32)),
+                         redo.blocks ? kLastResortWarps : uint32_t(gi->num_sms) * 4);
+    if (r != HNSW_OK) return r;
     if (a.persistent && warp_route) {
         uint32_t warps = 0;
         CU(persistent_warps(geo, gi->view.dp, gi->view.dc, gi->num_sms, &warps), "occupancy");
@@ -343,7 +356,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     // list never holds more entries than there are nodes; a query whose warp
     // finds the pool empty moves on to the next pass.
     const uint32_t tab_cap = (gi->view.n + kColdChunk - 1) / kColdChunk + 2;
-    {
+    if (geo.cold || !redo.blocks) {
         const uint32_t slots = geo.cold ? std::max(a.spill_slots, s->g_warps) : s->g_warps;
         const uint64_t want = std::max<uint64_t>((uint64_t(gi->view.n) * 8 + kColdChunk - 1) / kColdChunk,
                                                  uint64_t(slots) * 32);
@@ -381,16 +394,22 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         a.planned = s->planned.as<uint8_t>();
     }
     if (warp_route) CU(launch_search(a, geo, gi->num_sms, stream), "search kernel");
-    if (team.blocks) {
-        SearchArgs ta = a;
-        if (!team.bitmap_words) {
-            ta.spill_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
-            ta.spill_bits = s->team_bits.as<uint32_t>();
-        }
-        ta.team_far = s->team_far.as<uint64_t>();
-        CU(launch_search_team(ta, team, stream), "search team kernel");
+    SearchArgs ta = a;
+    ta.spill_words = bit_words;
+    ta.spill_bits = s->team_bits.as<uint32_t>();
+    ta.team_far = s->team_far.as<uint64_t>();
+    if (team.blocks) CU(launch_search_team(ta, team, stream), "search team kernel");
+    if (redo.blocks) {
+        ta.route = nullptr;
+        ta.order = a.overflow_list;
+        ta.team_count = a.overflow_count;
+        ta.work_next = s->work.as<uint32_t>() + 6;
+        ta.overflow_list = a.overflow_list2;
+        ta.overflow_count = a.overflow_count2;
+        CU(launch_search_team(ta, redo, stream), "search team retry kernel");
+    } else {
+        CU(launch_search_retry(a, s->g_warps, stream), "search retry kernel");
     }
-    CU(launch_search_retry(a, s->g_warps, stream), "search retry kernel");
     SearchArgs last = a;
     last.overflow_list = a.overflow_list2;
     last.overflow_count = a.overflow_count2;

@@ -119,6 +119,7 @@ struct SearchArgs {
     // takes the batch when the device decides (null: the one launched).
     const uint32_t* order = nullptr;
     const uint32_t* route = nullptr;
+    const uint32_t* team_count = nullptr;  // team kernel as a retry pass: the queries of `order`
     // Fallback workspaces in global memory (retry kernel only).
     uint64_t* g_results = nullptr;
     uint64_t* g_cands = nullptr;

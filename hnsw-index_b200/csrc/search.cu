@@ -73,14 +73,16 @@ static bool single_array_batch(const SearchArgs& args, const SearchGeometry& g) 
            g.cand_cap >= g.ef_cap + 32;
 }
 
-// Whether a single-array batch takes the kernels of 96 registers: its queries
-// fill the 16 warps per SM that 128 registers allow more than twice, and its
-// scratch (with the 1 KB the system takes per block) leaves room for more
-// warps. (10,000 queries: 1.00-1.16 times faster over 12 kinds of batch; 4,000:
-// 0.95-1.12.)
+// Whether a single-array batch takes the kernels of 96 registers: its scratch
+// (with the 1 KB the system takes per block) lets more than the 16 warps per SM
+// of 128 registers in, and its queries are just too many for one round of 16
+// or fill two. 2,500 queries: 0.95-1.23 times faster (int8 on 200k x 96, ef =
+// 48: 372 and 302 us), 10,000: 1.00-1.16; in between, 4,000, 0.95-1.12.
 static bool use_lean_kernel(uint32_t nq, const SearchGeometry& g, int num_sms) {
     const size_t block = size_t(g.bytes_per_warp) * g.warps_per_block + 1024;
-    return nq > 32u * uint32_t(num_sms) && size_t(228) * 1024 / block * g.warps_per_block > 16;
+    const uint32_t warps = std::min<uint32_t>(21, uint32_t(size_t(228) * 1024 / block * g.warps_per_block));
+    const uint32_t sms = uint32_t(num_sms);
+    return warps > 16 && nq > 16 * sms && (nq <= warps * sms || nq > 32 * sms);
 }
 
 // The search kernel a batch takes: the single-array variant when it applies,

@@ -919,12 +919,13 @@ __global__ void __launch_bounds__(512, 1) search_team_kernel(SearchArgs a, TeamG
     w.chk = a.chk;
 #endif
     TeamCtl& ctl = team_ctl(t);
+    const uint32_t queries = a.team_count ? *a.team_count : a.nq;
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) ctl.qi = atomicAdd(a.work_next, 1u);
         __syncthreads();
         uint32_t qi = ctl.qi;
-        if (qi >= a.nq) break;
+        if (qi >= queries) break;
         if (a.order) qi = a.order[qi];
         const int32_t st = team_query<DK>(a, w, t, qi);
         if (st == ST_OVERFLOW && threadIdx.x == 0) {

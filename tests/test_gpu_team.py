@@ -59,6 +59,22 @@ def test_team_batches_around_the_rule(nq):
     assert_same(gi.search_arrays(q[:nq], 10, 48), oi.search(q[:nq], 10, 48), f"nq={nq}")
 
 
+@pytest.mark.parametrize("ef", [32, 200])
+def test_team_retry_of_queries_that_outgrow_a_warp(ef):
+    """Plain warps whose visited hash fills (2048 slots at ef = 32, 16,384 at
+    200) hand the query to the teams' retry pass."""
+    base, q = H.gaussian(30000, 700, 64, 9)
+    b = H.IndexBuilder(64, H.Metric.L2, H.HnswParams(m=32, ef_construction=60, seed=7))
+    b.insert_batch_gpu(np.arange(30000, dtype=np.uint64), base)
+    data = b.to_bytes()
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    gi.set_counters(True)
+    got = gi.search_arrays(q, 10, ef, mode=0)
+    if ef == 32:
+        assert gi.read_counters(700)[:, 0].max() > 1536
+    assert_same(got, oi.search(q, 10, ef), f"ef={ef}")
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("sel", [0.02, 0.9])
 def test_batches_routed_on_the_device(mode, sel):
