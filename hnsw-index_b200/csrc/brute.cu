@@ -120,6 +120,26 @@ __device__ __forceinline__ bool brute_admits(const BruteArgs& a, uint32_t q, uin
     return bit < a.filter_nbits && ((__ldg(bits + (bit >> 6)) >> (bit & 63)) & 1ull);
 }
 
+// The rows that one filter for the whole batch admits, in any order: the score
+// kernel then reads and scores only those. (100 queries x 50k x 100 rows with
+// 20 % admitted: testing the bit after scoring every row took 229 us a call.)
+__global__ void __launch_bounds__(256) brute_rows_kernel(BruteArgs a) {
+    __shared__ uint32_t base, wcount[8];
+    const uint32_t r = blockIdx.x * 256 + threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool in = r < a.n && brute_admits(a, 0, r);
+    const uint32_t M = __ballot_sync(kFull, in);
+    if (lane == 0) wcount[warp] = __popc(M);
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (uint32_t w = 0; w < 8; ++w) {
+        before += w < warp ? wcount[w] : 0u;
+        all += wcount[w];
+    }
+    if (threadIdx.x == 0 && all) base = atomicAdd(a.row_list, all);
+    __syncthreads();
+    if (in) a.row_list[1 + base + before + __popc(M & ((1u << lane) - 1u))] = r;
+}
+
 // Two f32 operations per instruction, each rounded as its scalar form.
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t r;
@@ -228,7 +248,17 @@ __device__ __forceinline__ uint32_t kth_bound(const uint32_t (&v)[M], uint32_t k
 // pairs see disjoint rows, so the kk-th smallest of their minima bounds the
 // kk-th distance of all. They are published and read after 1, 3, 7, ... tiles
 // (a reader may see some of them late: every value is a real row's distance).
-template <bool L2, class T>
+//
+// What bounds it: instruction issue. A tile of 64 pairs at D = 128 takes 656
+// instructions, of them 284 packed FMAs and additions (the FMA pipe is 52 %
+// busy), 67 shared loads and 63 shuffles. 1,000 queries x 100k x 128 (L2, k =
+// 10): 1.66 ms; with scalar FMAs on 4 x 8 pairs, copies that did not overlap
+// and single insertions 3.47 ms; eight lanes per pair (16-byte shared loads)
+// 1.95 ms, bound by the shared-memory pipe, which serves a quarter warp at a
+// time; 16 rows per warp 2.34 ms, eight warps per SM not hiding latency; three
+// blocks per SM instead of four 1.72 ms.
+// LIST: the rows of a.row_list instead of all.
+template <bool L2, class T, bool LIST>
 __global__ void __launch_bounds__(T::kThreads, T::kThreads == 128 ? 4 : 8) brute_score_kernel(BruteArgs a, uint32_t kk,
                                                                                             uint32_t rows_per,
                                                                                             uint32_t nslices) {
@@ -248,7 +278,11 @@ __global__ void __launch_bounds__(T::kThreads, T::kThreads == 128 ? 4 : 8) brute
     uint2* meta = reinterpret_cast<uint2*>(reinterpret_cast<char*>(bufs) + T::kBufBytes);  // per list: (n, cnt)
     uint64_t* lists = reinterpret_cast<uint64_t*>(meta + T::kWarps * QW);
     const uint32_t q0 = blockIdx.x * T::QB, slice = blockIdx.y;
-    const uint32_t r_begin = min(a.n, slice * rows_per), r_end = min(a.n, r_begin + rows_per);
+    // Positions of the row list (its count first) when there is one, else rows.
+    const uint32_t* list = LIST ? a.row_list + 1 : nullptr;
+    const uint32_t nrows = LIST ? *a.row_list : a.n;
+    if (LIST) rows_per = ((nrows + nslices - 1) / nslices + T::RB - 1) / T::RB * T::RB;
+    const uint32_t r_begin = min(nrows, slice * rows_per), r_end = min(nrows, r_begin + rows_per);
     const uint32_t wq0 = q0 + uint32_t(wq * QW);  // this warp's first query
     const bool active = wq0 < a.nq;
     uint64_t* wbuf = bufs + size_t(warp) * QW * 32;
@@ -284,21 +318,37 @@ __global__ void __launch_bounds__(T::kThreads, T::kThreads == 128 ? 4 : 8) brute
     const uint32_t who = T::kPrivate ? uint32_t(lane) : threadIdx.x;
     const uint32_t my_c = (who % P) * 4, my_r = (T::kPrivate ? uint32_t(wr * RW) : 0u) + who / P;
     uint32_t issued = 0, kc_next = 0, row_next = r_begin + my_r, s_next = 0;
+    constexpr uint32_t kStep = (T::kPrivate ? 32 : T::kThreads) / P, kRows = (T::kPrivate ? RW : T::RB) / kStep;
+    // The rows of the next tile to copy (a tile ahead, so that a list's entries
+    // have arrived when the copies need them).
+    uint32_t ids[kRows], ids_next[kRows];
+    auto tile_ids = [&](uint32_t row0, uint32_t (&out)[kRows]) {
+#pragma unroll
+        for (uint32_t i = 0; i < kRows; ++i) out[i] = __ldg(list + min(row0 + i * kStep, r_end - 1));
+    };
+    if (LIST && total) {
+        tile_ids(row_next, ids);
+        tile_ids(row_next + T::RB, ids_next);
+    }
     auto advance = [&]() {
         if (issued < total) {
             const uint32_t col = kc_next * T::KC + my_c;
             if (col < dp) {
                 float* dst = sr + (s_next * T::RB + my_r) * T::kRowStride + my_c;
 #pragma unroll
-                for (uint32_t r = 0; r < uint32_t(T::kPrivate ? RW : T::RB);
-                     r += (T::kPrivate ? 32 : T::kThreads) / P) {
-                    const uint32_t row = min(row_next + r, r_end - 1);
-                    cp_async16(dst + r * T::kRowStride, a.base + size_t(row) * dp + col);
+                for (uint32_t i = 0; i < kRows; ++i) {
+                    const uint32_t row = LIST ? ids[i] : min(row_next + i * kStep, r_end - 1);
+                    cp_async16(dst + i * kStep * T::kRowStride, a.base + size_t(row) * dp + col);
                 }
             }
             if (++kc_next == nk) {
                 kc_next = 0;
                 row_next += T::RB;
+                if (LIST) {
+#pragma unroll
+                    for (uint32_t i = 0; i < kRows; ++i) ids[i] = ids_next[i];
+                    tile_ids(row_next + T::RB, ids_next);
+                }
             }
             s_next = s_next + 1 == T::kStages ? 0 : s_next + 1;
             ++issued;
@@ -409,7 +459,7 @@ __global__ void __launch_bounds__(T::kThreads, T::kThreads == 128 ? 4 : 8) brute
         thr = min(thr, shared_thr);
         bool want0 = dk0 <= thr && row0 < r_end && q < a.nq;
         bool want1 = dk1 <= thr && row0 + 1 < r_end && q < a.nq;
-        if (a.filter_bits) {
+        if (!LIST && a.filter_bits) {
             want0 = want0 && brute_admits(a, q, row0);
             want1 = want1 && brute_admits(a, q, row0 + 1);
         }
@@ -421,7 +471,7 @@ __global__ void __launch_bounds__(T::kThreads, T::kThreads == 128 ? 4 : 8) brute
 #pragma unroll 1
         for (uint32_t v = 0; v < 2; ++v) {
             const bool want = v ? want1 : want0;
-            const uint32_t row = row0 + v;
+            const uint32_t row = LIST && want ? __ldg(list + row0 + v) : row0 + v;
             uint64_t e = (uint64_t(v ? dk1 : dk0) << 32) | row;
             if (want && a.krank) e = (e & 0xFFFFFFFF00000000ull) | __ldg(a.krank + row);
             uint32_t W = __ballot_sync(kFull, want);
@@ -683,8 +733,10 @@ cudaError_t launch_brute_rerank(const BruteArgs& a, const uint64_t* cand, const 
 namespace {
 
 // The score kernel's shapes. A warp of eight queries x eight rows is the
-// general one; batches of one or two queries take QW = 2 so that the padding
-// is not computed, and small batches put more of the block's warps on rows.
+// general one. One or two queries take QW = 2 x 32 rows, so that six or seven
+// padding queries are not computed and more rows are in flight (one query x
+// 200k x 128: 41 us, 57 us with eight queries per warp). Up to eight queries
+// put all four warps on rows, up to 16 two: a warp without a query would idle.
 using TilePair = dev::BruteTile<2, 32, 1, 4>;
 using TileSmall = dev::BruteTile<8, 8, 1, 4>;
 using TileMid = dev::BruteTile<8, 8, 2, 2>;
@@ -699,22 +751,28 @@ struct BrutePlan {
 
 constexpr size_t kBruteSmemMax = 227 * 1024;
 
+template <class T, bool LIST>
+const void* score_kernel_of(bool l2) {
+    return l2 ? reinterpret_cast<const void*>(dev::brute_score_kernel<true, T, LIST>)
+              : reinterpret_cast<const void*>(dev::brute_score_kernel<false, T, LIST>);
+}
+
 template <class T>
-bool take_tile(BrutePlan& p, uint32_t dp, uint32_t list_kk, bool l2) {
+bool take_tile(BrutePlan& p, uint32_t dp, uint32_t list_kk, bool l2, bool rows) {
     const size_t s = T::smem(dp, list_kk);
     if (s > kBruteSmemMax) return false;
     p.qb = T::QB;
     p.rb = T::RB;
     p.threads = T::kThreads;
     p.smem = s;
-    p.kern = l2 ? reinterpret_cast<const void*>(dev::brute_score_kernel<true, T>)
-                : reinterpret_cast<const void*>(dev::brute_score_kernel<false, T>);
+    p.kern = rows ? score_kernel_of<T, true>(l2) : score_kernel_of<T, false>(l2);
     return true;
 }
 
-// Shape and row slices of a batch; at most max_slices lists per query.
+// Shape and row slices of a batch (`rows`: over a row list); at most
+// max_slices lists per query.
 cudaError_t plan_brute(uint32_t nq, uint32_t n, uint32_t dp, uint32_t k, int metric, int num_sms, uint32_t max_slices,
-                       BrutePlan* out) {
+                       bool rows, BrutePlan* out) {
     BrutePlan p;
     p.kk = std::max<uint32_t>(1, std::min<uint32_t>(k, n ? n : 1));
     *out = p;
@@ -724,12 +782,12 @@ cudaError_t plan_brute(uint32_t nq, uint32_t n, uint32_t dp, uint32_t k, int met
     const bool l2 = metric == 0;
     bool ok = false;
     if (p.kk <= dev::kSharedListMax) {
-        if (nq <= 2) ok = take_tile<TilePair>(p, dp, p.kk, l2);
-        if (!ok && nq > 16) ok = take_tile<TileBatch>(p, dp, p.kk, l2);
-        if (!ok && nq > 8) ok = take_tile<TileMid>(p, dp, p.kk, l2);
-        if (!ok) ok = take_tile<TileSmall>(p, dp, p.kk, l2);
+        if (nq <= 2) ok = take_tile<TilePair>(p, dp, p.kk, l2, rows);
+        if (!ok && nq > 16) ok = take_tile<TileBatch>(p, dp, p.kk, l2, rows);
+        if (!ok && nq > 8) ok = take_tile<TileMid>(p, dp, p.kk, l2, rows);
+        if (!ok) ok = take_tile<TileSmall>(p, dp, p.kk, l2, rows);
     } else {
-        ok = take_tile<TileLong>(p, dp, 0, l2);
+        ok = take_tile<TileLong>(p, dp, 0, l2, rows);
     }
     if (!ok) return cudaErrorInvalidValue;
     cudaError_t e = raise_smem_limit(p.kern);
@@ -762,7 +820,7 @@ int current_sms() {
 
 cudaError_t brute_slices(uint32_t nq, uint32_t n, uint32_t dp, uint32_t k, int metric, uint32_t* slices) {
     BrutePlan p;
-    cudaError_t e = plan_brute(nq, n, dp, k, metric, current_sms(), ~0u, &p);
+    cudaError_t e = plan_brute(nq, n, dp, k, metric, current_sms(), ~0u, false, &p);
     *slices = std::max<uint32_t>(p.slices, 1);
     return e;
 }
@@ -772,13 +830,20 @@ cudaError_t launch_brute_fp32(const BruteArgs& a, cudaStream_t stream) {
     BrutePlan p;
     if (empty) p.kk = p.slices = 1;
     else {
-        cudaError_t e = plan_brute(a.nq, a.n, a.dp, a.k, a.metric, current_sms(), a.tiles, &p);
+        cudaError_t e = plan_brute(a.nq, a.n, a.dp, a.k, a.metric, current_sms(), a.tiles, a.row_list != nullptr, &p);
         if (e != cudaSuccess) return e;
     }
     dev::brute_prep_kernel<<<(a.nq * 32 + 127) / 128, 128, 0, stream>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (!empty) {
+        if (a.row_list) {
+            e = cudaMemsetAsync(a.row_list, 0, 4, stream);
+            if (e != cudaSuccess) return e;
+            dev::brute_rows_kernel<<<(a.n + 255) / 256, 256, 0, stream>>>(a);
+            e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+        }
         uint32_t rows_per = ((a.n + p.slices - 1) / p.slices + p.rb - 1) / p.rb * p.rb;
         p.slices = (a.n + rows_per - 1) / rows_per;
         BruteArgs b = a;

@@ -1420,6 +1420,12 @@ static int brute_search_fp32(hnsw_gpu_brute* b, const float* queries, size_t nq,
             CU(cudaMemcpyAsync(b->fused.p, f->used, nq, cudaMemcpyHostToDevice, st), "copy filter flags");
             a.filter_used = b->fused.as<uint8_t>();
         }
+        // One bitmap for every query: score the rows it admits only. (Without
+        // memory for their list the score kernel tests the bits.)
+        if (!f->stride && !f->used && b->n) {
+            if (b->rows.ensure((size_t(b->n) + 1) * 4) == cudaSuccess) a.row_list = b->rows.as<uint32_t>();
+            else cudaGetLastError();
+        }
     }
     CU(launch_brute_fp32(a, st), "brute kernel");
     CU(b->out.fetch(st, out_keys, out_dist, out_count, out_status, k != 0), "brute search");

@@ -299,7 +299,7 @@ struct hnsw_gpu_brute {
     std::mutex mu;
     DBuf qprep, part, minima, q;
     hnswgpu::Outputs out;
-    DBuf fbits, fused, fids;  // filter bitmaps, flags and bitmap ids of a filtered search
+    DBuf fbits, fused, fids, rows;  // filter bitmaps, flags, bitmap ids and admitted rows of a filtered search
     // Tensor-core path: BF16 operand rows per term count (index 0: 1 term, 1: 3 terms).
     DBuf bop[2], xnorm2;
     uint32_t bop_kp[2] = {0, 0};
@@ -313,7 +313,7 @@ struct hnsw_gpu_brute {
     cudaStream_t stream = nullptr;
     ~hnsw_gpu_brute() {
         DeviceGuard g(device);
-        for (DBuf* b : {&base, &keys, &krank, &skeys, &qprep, &part, &minima, &q, &fbits, &fused, &fids,
+        for (DBuf* b : {&base, &keys, &krank, &skeys, &qprep, &part, &minima, &q, &fbits, &fused, &fids, &rows,
                         &bop[0], &bop[1], &xnorm2,
                         &aop, &dense, &thr1, &thr2, &margin, &qnorm2, &cand})
             b->release();

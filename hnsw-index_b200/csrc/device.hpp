@@ -284,6 +284,9 @@ struct BruteArgs {
     const uint8_t* filter_used = nullptr;
     const uint32_t* filter_ids = nullptr;
     int filter_by_row = 0;
+    // Scratch for one filter shared by the batch (n + 1 words, or null): the
+    // count and the rows it admits; the others are then not read.
+    uint32_t* row_list = nullptr;
 };
 cudaError_t launch_brute_fp32(const BruteArgs& a, cudaStream_t stream);
 // Row slices (lists per query) that a batch is cut into when nothing limits
