@@ -57,6 +57,8 @@ constexpr uint32_t kTeamBins = 1024;              // histogram of a refill
 // Block-wide state.
 struct TeamCtl {
     uint64_t E[kTeamNew], EA[kTeamNew];     // merged neighbors, and the admitted ones (~0: none)
+    uint64_t seq[kTeamNew];                 // the lists' improving neighbors in order, repeats included
+    uint32_t seq_adm[kTeamNew];             // whether each is admitted
     uint64_t fmin, fmax;                    // far list: smallest entry; refill window
     uint32_t lmin[kTeamLists];              // per leading candidate: smallest unvisited neighbor (order_key)
     uint32_t lcnt[kTeamLists];              // its improving neighbors, admitted ones << 16
@@ -633,6 +635,8 @@ __device__ __forceinline__ int32_t team_query(const SearchArgs& a, Ws& w, const 
                         const uint32_t e = at + __popc(imp[h] & ((1u << lane) - 1u));
                         ctl.E[e] = fresh ? x : ~0ull;
                         ctl.EA[e] = fresh && inA ? x : ~0ull;
+                        ctl.seq[e] = x;
+                        ctl.seq_adm[e] = inA ? 1u : 0u;
                     }
                     at += __popc(imp[h]);
                     const uint32_t nC = __popc(__ballot_sync(kFull, in && fresh && x <= fmin));
@@ -738,15 +742,18 @@ __device__ __forceinline__ int32_t team_query(const SearchArgs& a, Ws& w, const 
                 one_by_one = __syncthreads_or(rs + new_r >= ef && tie != 0 && tie >= order_key(R2[ef - 1]));
             if (one_by_one) {
                 // Warp 0 takes the new entries one by one on the old copies
-                // (the far list as it was).
+                // (the far list as it was), each where the lists have it
+                // first: of lists that share a neighbor, any may have marked it.
                 if (warp == 0) {
                     uint64_t* Cw = team_C(t, b);
                     uint64_t* Rw = team_R(t, b);
                     uint32_t tl = tail, r = rs, fc = fcount;
                     uint64_t fm = fcount ? fmin : ~0ull;
                     for (uint32_t e = 0; e < ne; ++e) {
-                        const uint64_t x = ctl.E[e];
-                        if (x == ~0ull) continue;
+                        const uint64_t x = ctl.seq[e];
+                        bool repeat = false;
+                        for (uint32_t f = lane; f < e; f += 32) repeat |= ctl.seq[f] == x;
+                        if (__any_sync(kFull, repeat)) continue;
                         if (r >= ef && !(pdist(x) < pdist(Rw[r - 1]))) continue;
                         uint64_t to_far = ~0ull;
                         if (fc && x > fm) {
@@ -768,7 +775,7 @@ __device__ __forceinline__ int32_t team_query(const SearchArgs& a, Ws& w, const 
                             ++fc;
                             fm = min(fm, to_far);
                         }
-                        if (ctl.EA[e] != ~0ull) {
+                        if (ctl.seq_adm[e]) {
                             sorted_insert(Rw, 0, r, x);
                             r = min(r + 1, ef);
                         }

@@ -102,3 +102,20 @@ def test_team_with_its_visited_bitmap_in_global_memory():
     bits = H.key_bitmap(np.arange(0, n, 3, dtype=np.uint64), n)
     kw = dict(filter_bits=bits, filter_nbits=n)
     assert_same(gi.search_arrays(q, 10, 40, **kw), oi.search(q, 10, 40, **kw), "filtered")
+
+
+@pytest.mark.parametrize("quantized", [False, True])
+def test_team_ties_at_the_worst_result_across_lists(quantized):
+    """A few hundred distinct distances among 20,000 nodes: neighbors shared by
+    the lists of one joint expansion tie with the worst result, so the order
+    of the lists decides (whichever list marked the neighbor)."""
+    rng = np.random.default_rng(12)
+    base = rng.integers(-8, 9, (20000, 4)).astype(np.float32)
+    q = rng.integers(-8, 9, (2368, 4)).astype(np.float32)
+    data = build_index(base, m=16, ef_construction=60, quantize=True)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    for ef in (20, 64):
+        ref = oi.search(q, 10, ef, quantized=quantized)
+        for lo in range(0, len(q), 296):
+            got = gi.search_arrays(q[lo:lo + 296], 10, ef, quantized=quantized)
+            assert_same(got, tuple(x[lo:lo + 296] for x in ref), f"ef={ef} from {lo}")
