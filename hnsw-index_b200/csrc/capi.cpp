@@ -787,6 +787,7 @@ static int stage_batch(Slot* s, const float* queries, size_t nq, size_t dim, con
         }
     }
     CU(s->out.ensure(nq, stride), "cudaMalloc outputs");
+    if (o.ks || o.filter_bits) CU(s->out.clear(st), "clear outputs");
     out->ks = d_ks;
     out->efs = d_efs;
     out->fbits = d_fb;
@@ -1392,6 +1393,7 @@ static int brute_search_fp32(hnsw_gpu_brute* b, const float* queries, size_t nq,
     CU(b->minima.ensure(nq * kBruteMinima * 4), "cudaMalloc lane minima");
     a.minima = b->minima.as<uint32_t>();
     CU(b->out.ensure(nq, kk), "cudaMalloc outputs");
+    if (f && f->bits) CU(b->out.clear(st), "clear outputs");
     a.queries = b->q.as<float>();
     a.qprep = b->qprep.as<float>();
     a.part = b->part.as<uint64_t>();

@@ -98,6 +98,9 @@ struct Outputs {
         tail = extra_bytes;
         return dev.ensure(std::max<size_t>(bytes(), 16));
     }
+    // Zeroes the rows of a call that may fill them in part: the buffer holds
+    // what another call, of another shape, left there.
+    cudaError_t clear(cudaStream_t st) { return cudaMemsetAsync(dev.p, 0, rows * stride * 12, st); }
     // Enqueues the copies, waits for the stream, and fills the caller's arrays
     // (`extra_out` with the extra bytes; `rows_out` false: no keys and distances).
     cudaError_t fetch(cudaStream_t st, uint64_t* k, float* d, uint32_t* c, int32_t* s, bool rows_out = true,

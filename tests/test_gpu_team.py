@@ -119,3 +119,18 @@ def test_team_ties_at_the_worst_result_across_lists(quantized):
         for lo in range(0, len(q), 296):
             got = gi.search_arrays(q[lo:lo + 296], 10, ef, quantized=quantized)
             assert_same(got, tuple(x[lo:lo + 296] for x in ref), f"ef={ef} from {lo}")
+
+
+def test_entries_beyond_the_counts_are_zero():
+    """Rows that a call fills in part (an uneven k, a filter of few rows) keep
+    nothing of an earlier call's of another shape."""
+    base, q = H.mixture(3000, 400, 24, 20, 0.4, 5)
+    gi = H.HnswIndex.from_bytes(build_index(base, m=8, ef_construction=40))
+    few = H.key_bitmap(np.arange(0, 3000, 1000, dtype=np.uint64), 3000)
+    kw = dict(filter_bits=few, filter_nbits=3000)
+    for nq in (400, 40):
+        gi.search_arrays(q, 20, 64)
+        ks = (np.arange(nq) % 10 + 1).astype(np.uint32)
+        for r in (gi.search_arrays(q[:nq], 10, 64, ks=ks), gi.search_arrays(q[:nq], 10, 64, **kw)):
+            beyond = np.arange(r[0].shape[1])[None, :] >= r[2][:, None]
+            assert beyond.any() and not r[0][beyond].any() and not r[1][beyond].any()
