@@ -288,13 +288,11 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     // A team of warps per query where one warp each would leave the batch
     // waiting on memory latency: up to two teams per SM, or four when the
     // queries are alike. Larger batches of unlike queries (filters, an ef per
-    // query) are decided on the device from their expected work, except a
-    // request loop's, whose short requests would wait for the long ones ahead
-    // of them.
+    // query) are decided on the device from their expected work.
     TeamGeometry team;
     const bool plans = o.exact_below > 0.0f && d_fbits, varied = d_efs || d_fbits;
     const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
-    if (heuristic && !o.traversal && !plans && tags == 0 && (small || (varied && !publish)))
+    if (heuristic && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
     // Without memory for the teams the batch takes the warp kernels.
     const uint32_t bit_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
