@@ -84,6 +84,16 @@ def test_wide_rows_and_large_m0():
     assert gpu_build(base, H.Metric.Cosine, params, max_wave=1).to_bytes() == want
 
 
+@pytest.mark.parametrize("metric", [H.Metric.L2, H.Metric.InnerProduct])
+@pytest.mark.parametrize("m,m0,dim", [(4, 5, 33), (8, 9, 37), (16, 17, 40), (8, 33, 45), (32, 65, 31)])
+def test_list_widths_around_the_rows_in_flight(metric, m, m0, dim):
+    """Lists of one entry more than 4, 8, 16, 32 and 64 rows; ragged dims."""
+    base, _ = H.mixture(600, 0, dim, 8, 0.4, m0)
+    params = H.HnswParams(m=m, m0=m0, ef_construction=70, seed=13)
+    want = cpu_sequential(base, metric, params).to_bytes()
+    assert gpu_build(base, metric, params, max_wave=1).to_bytes() == want
+
+
 def test_upper_layers_with_small_level_multiplier_base():
     # mL = 1 / ln 2: about half the nodes above layer 0, many promotions.
     base, _ = H.gaussian(800, 0, 12, 31)
