@@ -747,8 +747,19 @@ __device__ __forceinline__ int32_t team_query(const SearchArgs& a, Ws& w, const 
                 if (warp == 0) {
                     uint64_t* Cw = team_C(t, b);
                     uint64_t* Rw = team_R(t, b);
-                    uint32_t tl = tail, r = rs, fc = fcount;
+                    uint32_t tl = ncj, r = rs, fc = fcount;
                     uint64_t fm = fcount ? fmin : ~0ull;
+                    // C's live range moves to its start first: these merges
+                    // do not reset `head`, so many in a row would run the
+                    // range out of the array, down to an empty one at its end.
+                    if (head > 0)
+                        for (uint32_t i0 = 0; i0 < ncj; i0 += 32) {
+                            const uint32_t i = i0 + uint32_t(lane);
+                            const uint64_t v = i < ncj ? Cw[head + i] : 0ull;
+                            __syncwarp();
+                            if (i < ncj) Cw[i] = v;
+                            __syncwarp();
+                        }
                     for (uint32_t e = 0; e < ne; ++e) {
                         const uint64_t x = ctl.seq[e];
                         bool repeat = false;
@@ -758,16 +769,16 @@ __device__ __forceinline__ int32_t team_query(const SearchArgs& a, Ws& w, const 
                         uint64_t to_far = ~0ull;
                         if (fc && x > fm) {
                             to_far = x;
-                        } else if (tl - head >= t.cap || tl >= t.cap + 31) {
+                        } else if (tl >= t.cap) {
                             to_far = Cw[tl - 1];  // the largest leaves C
                             __syncwarp();
                             if (x > to_far) {
                                 to_far = x;
                             } else {
-                                sorted_insert(Cw, head, tl - 1, x);
+                                sorted_insert(Cw, 0, tl - 1, x);
                             }
                         } else {
-                            sorted_insert(Cw, head, tl, x);
+                            sorted_insert(Cw, 0, tl, x);
                             ++tl;
                         }
                         if (to_far != ~0ull) {
@@ -789,6 +800,7 @@ __device__ __forceinline__ int32_t team_query(const SearchArgs& a, Ws& w, const 
                     }
                 }
                 __syncthreads();
+                head = 0;
                 tail = ctl.tail;
                 rs = ctl.rs;
             } else {

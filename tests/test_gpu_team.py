@@ -5,6 +5,8 @@ queue's far list, equal distances everywhere (small integers), deleted nodes,
 a visited bitmap in global memory, and batches routed on the device. Keys,
 distance bits, counts and statuses are equal (no tolerance)."""
 
+import struct
+
 import numpy as np
 import pytest
 
@@ -134,3 +136,31 @@ def test_entries_beyond_the_counts_are_zero():
         for r in (gi.search_arrays(q[:nq], 10, 64, ks=ks), gi.search_arrays(q[:nq], 10, 64, **kw)):
             beyond = np.arange(r[0].shape[1])[None, :] >= r[2][:, None]
             assert beyond.any() and not r[0][beyond].any() and not r[1][beyond].any()
+
+
+@pytest.mark.parametrize("every", [1, 4])
+def test_merges_of_ties_in_a_row(every):
+    """A chain of 250 levels, each two points at one distance (x and -x), the
+    first listing the next level: each merge is taken one by one and the next
+    expansion empties the queue, more often than its array (128) is long."""
+    levels, n = 250, 501
+    x = [float(levels + 1)]
+    lists = [[] for _ in range(n)]
+    for i in range(levels):
+        lists[max(2 * i - 1, 0)] = [2 * i + 1, 2 * i + 2]
+        x += [float(levels - i), -float(levels - i)]
+    head = bytearray(build_index(np.zeros((1, 1), np.float32), m=8, ef_construction=40)[:56])
+    struct.pack_into("<II", head, 48, n, 0)
+    body = (bytes(head) + np.arange(n, dtype="<u8").tobytes() + bytes(2 * n) + np.array(x, "<f4").tobytes()
+            + b"".join(struct.pack(f"<I{len(a)}I", len(a), *a) for a in lists))
+    data = body + struct.pack("<I", H.crc32(body))
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    q = np.zeros((1, 1), np.float32)
+    kw = {}
+    if every > 1:
+        bits = H.key_bitmap(np.array([i for i in range(n) if i % every < 3], np.uint64), n)
+        kw = dict(filter_bits=bits, filter_nbits=n)
+    for ef in (1, 5):
+        ref = oi.search(q, 1, ef, **kw)
+        assert ref[0][0, 0] == 499 or every > 1
+        assert_same(gi.search_arrays(q, 1, ef, **kw), ref, f"ef={ef} every={every}")
