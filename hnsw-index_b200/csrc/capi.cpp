@@ -294,19 +294,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
     if (heuristic && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
-    // Without memory for the teams the batch takes the warp kernels.
-    const uint32_t bit_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
-    auto ensure_team = [&](TeamGeometry& g) {
-        if (!g.blocks) return;
-        cudaError_t e = s->team_far.ensure(size_t(g.blocks) * g.far_cap * 8);
-        if (e == cudaSuccess && !g.bitmap_words) e = s->team_bits.ensure(size_t(g.blocks) * bit_words * 4);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            g = TeamGeometry();
-        }
-    };
-    ensure_team(team);
-    const bool warp_route = !team.blocks || !small;
+    bool warp_route = !team.blocks || !small;
     // Queries that outgrow a warp's scratch are redone by teams (one per SM):
     // a warp of the retry kernel takes milliseconds for one, and the batch
     // waits for it.
@@ -315,7 +303,22 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         SearchArgs one = a;
         one.nq = uint32_t(gi->num_sms);
         CU(plan_search_team(one, ef_max, gi->num_sms, &redo), "team occupancy");
-        ensure_team(redo);
+    }
+    // Both launches share the team buffers: each buffer grows once, to what
+    // the larger needs (growing it for one after the other would free what the
+    // first was planned with). Without memory for them the batch takes the
+    // warp kernels.
+    const uint32_t bit_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
+    if (team.blocks || redo.blocks) {
+        auto far = [](const TeamGeometry& g) { return size_t(g.blocks) * g.far_cap * 8; };
+        auto bits = [&](const TeamGeometry& g) { return g.bitmap_words ? 0 : size_t(g.blocks) * bit_words * 4; };
+        cudaError_t e = s->team_far.ensure(std::max(far(team), far(redo)));
+        if (e == cudaSuccess) e = s->team_bits.ensure(std::max(bits(team), bits(redo)));
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            team = redo = TeamGeometry();
+            warp_route = true;
+        }
     }
     int r = ensure_retry(gi, s, std::max(geo.ef_cap, round_up(ef_max, 32)),
                          redo.blocks ? kLastResortWarps : uint32_t(gi->num_sms) * 4);

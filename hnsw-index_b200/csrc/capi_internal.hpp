@@ -58,10 +58,10 @@ struct DBuf {
     size_t bytes = 0;
     cudaError_t ensure(size_t need) {
         if (need <= bytes) return cudaSuccess;
-        if (injected_alloc_failure()) return cudaErrorMemoryAllocation;  // buffer left as it was
         if (p) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        if (injected_alloc_failure()) return cudaErrorMemoryAllocation;  // as cudaMalloc: the old buffer is gone
         cudaError_t e = cudaMalloc(&p, need);
         if (e == cudaSuccess) bytes = need;
         return e;

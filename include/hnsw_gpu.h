@@ -371,8 +371,8 @@ int hnsw_gpu_brute_set_pairs(hnsw_gpu_brute* brute, int enabled);
 
 /* Test hook: the next `count` device allocations the library attempts fail
  * as cudaErrorMemoryAllocation would, so callers can exercise the
- * HNSW_ERR_OUT_OF_DEVICE_MEMORY paths (0 clears it). The failing call leaves
- * its handle as it was; later calls allocate normally. Process-wide. No
+ * HNSW_ERR_OUT_OF_DEVICE_MEMORY paths (0 clears it). The handle of the failing
+ * call stays usable; later calls allocate normally. Process-wide. No
  * counterpart in the reference. */
 void hnsw_gpu_debug_fail_allocations(int count);
 

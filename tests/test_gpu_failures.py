@@ -96,3 +96,28 @@ def test_allocation_failure_at_open_leaves_nothing_behind():
         H.debug_fail_allocations(0)
     gi = H.HnswIndex.from_bytes(data)
     assert gi.len() == 2000
+
+
+def test_team_buffers_that_cannot_grow_leave_the_batch_to_the_warp_kernels():
+    """A batch that may take teams and whose overflowing queries are redone by
+    teams plans both on one far list. Above 226,719 nodes the second needs a
+    little more than the first, so after a batch that allocated the first's
+    size exactly the buffer has to grow; when that fails neither may run."""
+    n, nq = 240_000, 900
+    base, q = H.mixture(n, nq, 4, 300, 0.3, 2)
+    b = H.IndexBuilder(4, H.Metric.L2, H.HnswParams(m=4, ef_construction=16, seed=7))
+    b.insert_batch_gpu(np.arange(n, dtype=np.uint64), base)
+    data = b.to_bytes()
+    gi = H.HnswIndex.from_bytes(data)
+    efs = np.random.default_rng(3).choice([16, 40, 64], nq).astype(np.uint32)
+    ref = O.Index(data).search(q, 10, 16, efs=efs)
+    gi.set_schedule(ef_cap=64, hash_cap=2048, warps_per_block=2)  # every buffer but the teams'
+    _same(gi.search_arrays(q, 10, 16, efs=efs), ref)
+    gi.set_schedule()
+    _same(gi.search_arrays(q[:296], 10, 16, efs=efs[:296]), tuple(x[:296] for x in ref))
+    try:
+        H.debug_fail_allocations(1)
+        _same(gi.search_arrays(q, 10, 16, efs=efs), ref)
+    finally:
+        H.debug_fail_allocations(0)
+    _same(gi.search_arrays(q, 10, 16, efs=efs), ref)
