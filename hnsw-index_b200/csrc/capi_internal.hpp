@@ -86,6 +86,7 @@ struct Outputs {
     DBuf dev;
     void* host = nullptr;
     size_t host_bytes = 0, rows = 0, stride = 0, tail = 0;
+    bool cleared = false;
     uint64_t* keys() const { return dev.as<uint64_t>(); }
     float* dist() const { return reinterpret_cast<float*>(keys() + rows * stride); }
     uint32_t* count() const { return reinterpret_cast<uint32_t*>(dist() + rows * stride); }
@@ -96,11 +97,26 @@ struct Outputs {
         rows = nq;
         stride = row_stride;
         tail = extra_bytes;
+        cleared = false;
         return dev.ensure(std::max<size_t>(bytes(), 16));
     }
-    // Zeroes the rows of a call that may fill them in part: the buffer holds
-    // what another call, of another shape, left there.
-    cudaError_t clear(cudaStream_t st) { return cudaMemsetAsync(dev.p, 0, rows * stride * 12, st); }
+    // The buffer holds what another call, of another shape, left there, so the
+    // entries beyond a row's count are zeroed: on the device before a call
+    // that will leave many (a k per query, a filter), else in the caller's
+    // arrays (few or none: rows with k above the number of live nodes, failed
+    // queries; the scan of 10,000 counts takes about 3 us).
+    cudaError_t clear(cudaStream_t st) {
+        cleared = true;
+        return cudaMemsetAsync(dev.p, 0, rows * stride * 12, st);
+    }
+    void zero_unfilled(uint64_t* k, float* d, const uint32_t* c, const int32_t* s) const {
+        for (size_t i = 0; i < rows; ++i) {
+            const size_t n = s[i] == HNSW_OK ? c[i] : 0;
+            if (n >= stride) continue;
+            std::memset(k + i * stride + n, 0, (stride - n) * 8);
+            std::memset(d + i * stride + n, 0, (stride - n) * 4);
+        }
+    }
     // Enqueues the copies, waits for the stream, and fills the caller's arrays
     // (`extra_out` with the extra bytes; `rows_out` false: no keys and distances).
     cudaError_t fetch(cudaStream_t st, uint64_t* k, float* d, uint32_t* c, int32_t* s, bool rows_out = true,
@@ -127,6 +143,7 @@ struct Outputs {
                 std::memcpy(c, at(count()), rows * 4);
                 std::memcpy(s, at(status()), rows * 4);
                 if (extra_out) std::memcpy(extra_out, at(extra()), tail);
+                if (rows_out && !cleared) zero_unfilled(k, d, c, s);
                 return cudaSuccess;
             }
         }
@@ -139,7 +156,9 @@ struct Outputs {
         copy(k, keys(), kb);
         copy(d, dist(), db);
         if (extra_out) copy(extra_out, extra(), tail);
-        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess && rows_out && !cleared) zero_unfilled(k, d, c, s);
+        return e;
     }
     void release() {
         dev.release();

@@ -138,6 +138,39 @@ def test_entries_beyond_the_counts_are_zero():
             assert beyond.any() and not r[0][beyond].any() and not r[1][beyond].any()
 
 
+
+@pytest.mark.parametrize("nq,k", [(40, 20), (700, 200)])
+def test_rows_of_any_call_are_zero_beyond_their_counts(nq, k):
+    """k above the number of points, and an invalid query, in graph and
+    brute-force searches of every precision, small results (one pinned copy)
+    and large ones, after a call that filled every row."""
+    base, q = H.mixture(3000, nq, 24, 20, 0.4, 5)
+    few = 15
+    gi = H.HnswIndex.from_bytes(build_index(base, m=8, ef_construction=40, deleted_keys=range(few, 3000)))
+    live = H.HnswIndex.from_bytes(build_index(base, m=8, ef_construction=40))
+    bf = H.BruteForceIndex(24, H.Metric.L2)
+    bf.insert_batch(np.arange(few, dtype=np.uint64), base[:few])
+    full = H.BruteForceIndex(24, H.Metric.L2)
+    full.insert_batch(np.arange(3000, dtype=np.uint64), base)
+    bad = q.copy()
+    bad[nq // 2, 3] = np.nan
+
+    def check(r):
+        filled = np.where(r[3] == 0, r[2], 0)
+        beyond = np.arange(r[0].shape[1])[None, :] >= filled[:, None]
+        assert beyond.any() and not r[0][beyond].any() and not r[1][beyond].any()
+
+    gi.search_arrays(q, few, 256)
+    check(gi.search_arrays(q, k, 256))
+    live.search_arrays(q, k, 256)
+    check(live.search_arrays(bad, k, 256, raise_on_error=False))
+    for precision in (H.Precision.FP32, H.Precision.BF16, H.Precision.BF16X3):
+        bf.search_arrays(q[:nq // 2], few, precision)
+        check(bf.search_arrays(q, k, precision))
+        full.search_arrays(q, few, precision)
+        check(full.search_arrays(bad, k, precision, raise_on_error=False))
+
+
 @pytest.mark.parametrize("every", [1, 4])
 def test_merges_of_ties_in_a_row(every):
     """A chain of 250 levels, each two points at one distance (x and -x), the
