@@ -149,9 +149,11 @@ static int ensure_retry(hnsw_gpu_index* gi, Slot* s, uint32_t ef_cap, uint32_t w
 
 // Enqueues one search on `stream` with device pointers. ef_max bounds every
 // per-query max(ef, k) of the batch.
-// The schedule comes from, in order: `force` (the autotuner's trials), the
-// fixed schedule, the tuning table, the occupancy heuristic. HNSW_MODE_AUTO
-// resolves to the tuned mode of the bucket, else persistent.
+// The schedule of the warp kernels comes from, in order: `force` (the
+// autotuner's trials; ef_cap 0 for the heuristic's), the fixed schedule, the
+// tuning table, the occupancy heuristic. HNSW_MODE_AUTO resolves to the tuned
+// mode of the bucket, else persistent. A batch may take teams under any but a
+// fixed schedule, which keeps it on the warp kernels, and a trial's.
 // Builds the tensor-core traversal rows on first use (and the low parts on
 // the first BF16X3 search). The build is waited for before the lock is
 // released, so a search on any stream that finds them ready can read them.
@@ -192,10 +194,13 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     const uint32_t tcb = o.traversal ? round_up(gi->view.dim, 32) * 2u * (o.traversal == HNSW_TRAVERSAL_BF16X3 ? 2u : 1u)
                                      : 0u;
     SearchGeometry geo{0, 0, 0, 0, 0};
+    bool teams = true, redo_teams = true;
     if (force) {
         geo = *force;
+        teams = geo.ef_cap == 0;
     } else if (gi->fixed.ef_cap) {
         geo = gi->fixed;
+        teams = redo_teams = false;
     } else {
         std::lock_guard<std::mutex> l(gi->tune_mu);
         const hnsw_gpu_index::Tuned& t = gi->tuned[tune_bucket(ef_max)];
@@ -292,14 +297,14 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     TeamGeometry team;
     const bool plans = o.exact_below > 0.0f && d_fbits, varied = d_efs || d_fbits;
     const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
-    if (heuristic && !o.traversal && !plans && tags == 0 && (small || varied))
+    if (teams && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
     bool warp_route = !team.blocks || !small;
     // Queries that outgrow a warp's scratch are redone by teams (one per SM):
     // a warp of the retry kernel takes milliseconds for one, and the batch
     // waits for it.
     TeamGeometry redo;
-    if (heuristic && !o.traversal && tags == 0 && warp_route && ef_max <= 1024) {
+    if (redo_teams && !o.traversal && tags == 0 && warp_route && ef_max <= 1024) {
         SearchArgs one = a;
         one.nq = uint32_t(gi->num_sms);
         CU(plan_search_team(one, ef_max, gi->num_sms, &redo), "team occupancy");
@@ -905,14 +910,18 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
         return x.ef_cap == y.ef_cap && x.cand_cap == y.cand_cap && x.hash_cap == y.hash_cap &&
                x.warps_per_block == y.warps_per_block && x.stage_rows == y.stage_rows && x.cold == y.cold;
     };
-    // Times one schedule; returns false on an error (status in r).
+    // Times one schedule; returns false on an error (status in r). The
+    // heuristic's is timed as a search on an untuned index runs (teams where
+    // the batch takes them), the others on the warp kernels alone.
+    const SearchGeometry automatic{0, 0, 0, 0, 0};
     auto timed = [&](const SearchGeometry& g, int32_t mode, int32_t heuristic, float* ms) {
         hnsw_search_opts ot = o;
         ot.mode = mode;
+        const SearchGeometry* force = heuristic ? &automatic : &g;
         auto run = [&]() {
             return enqueue_search(gi, s, s->q.as<float>(), nq, ot, sb.ks, sb.efs, sb.fbits, sb.fused, sb.fids,
                                   s->out.keys(), s->out.dist(), s->out.count(), s->out.status(), ef_bound, stride, st,
-                                  &g);
+                                  force);
         };
         r = run();  // warm-up; sizes every buffer
         if (r != HNSW_OK) return false;
@@ -993,8 +1002,7 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
     {
         std::lock_guard<std::mutex> l(gi->tune_mu);
         hnsw_gpu_index::Tuned& slot = gi->tuned[tune_bucket(ef_bound)];
-        slot.geo[0] = win[0]->g;
-        slot.geo[1] = win[1]->g;
+        for (int m : {0, 1}) slot.geo[m] = win[m]->heuristic ? automatic : win[m]->g;
         slot.mode = top->mode;
     }
     auto fill = [](const Trial& t, hnsw_tune_entry* e) {

@@ -182,8 +182,9 @@ void hnsw_gpu_graph_destroy(hnsw_gpu_graph* graph);
 /* Scratch geometry of the traversal kernel ("schedule"). By default the
  * library picks it per call from the batch's largest ef and the index's
  * dimension (results capacity, candidate capacity, visited-hash size, warps
- * per block chosen for the most resident warps). A fixed schedule overrides
- * that; NULL restores the automatic choice. Results do not depend on it. */
+ * per block chosen for the most resident warps), and whether a batch is
+ * searched by teams of warps. A fixed schedule overrides that (one warp per
+ * query); NULL restores the automatic choice. Results do not depend on it. */
 typedef struct hnsw_schedule {
     uint32_t ef_cap;          /* >= every max(ef, k) of a batch; multiple of 32, <= 1024 */
     uint32_t cand_cap;        /* candidate array entries */
@@ -207,11 +208,15 @@ int hnsw_gpu_set_schedule(hnsw_gpu_index* index, const hnsw_schedule* schedule);
  * mode x warps per block {1, 2, 4, 8} x visited-hash size {16, 32, 64} x
  * ef_cap (rounded up to a multiple of 64, 1024..32768 entries) x staged
  * rows, by coordinate descent from the heuristic's own choice, `reps` timed runs each after one warm-up (median,
- * CUDA events). The fastest schedule of each mode is stored in the index's
- * tuning table for the ef bucket of the sample's max(ef, k) (buckets of 32),
- * used from then on by searches in that bucket unless a fixed schedule is
- * set; HNSW_MODE_AUTO picks the faster mode. Results never depend on the
- * schedule. `entries` (optional, `cap` entries) receives every trial. */
+ * CUDA events). The heuristic's entry is timed as an untuned search runs (with
+ * a team of warps per query where the batch takes them), the others on the
+ * one-warp kernels. Unless the heuristic won, the fastest schedule of each
+ * mode is stored in the index's tuning table for the ef bucket of the sample's
+ * max(ef, k) (buckets of 32), used from then on by the one-warp kernels of
+ * searches in that bucket unless a fixed schedule is set (which also keeps
+ * every search on those kernels); HNSW_MODE_AUTO picks the faster mode.
+ * Results never depend on the schedule. `entries` (optional, `cap` entries)
+ * receives every trial. */
 typedef struct hnsw_tune_entry {
     hnsw_schedule schedule;
     int32_t mode;  /* HNSW_MODE_PLAIN or HNSW_MODE_PERSISTENT */

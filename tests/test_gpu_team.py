@@ -5,7 +5,9 @@ queue's far list, equal distances everywhere (small integers), deleted nodes,
 a visited bitmap in global memory, and batches routed on the device. Keys,
 distance bits, counts and statuses are equal (no tolerance)."""
 
+import statistics
 import struct
+import time
 
 import numpy as np
 import pytest
@@ -197,3 +199,26 @@ def test_merges_of_ties_in_a_row(every):
         ref = oi.search(q, 1, ef, **kw)
         assert ref[0][0, 0] == 499 or every > 1
         assert_same(gi.search_arrays(q, 1, ef, **kw), ref, f"ef={ef} every={every}")
+
+
+@pytest.mark.parametrize("sample", [1, 700])
+def test_a_tuned_index_keeps_its_teams(sample):
+    """Tuning picks the schedule of the one-warp kernels: one query of a tuned
+    bucket still takes a team (0.46 of one warp's time at ef = 256; the
+    limit of 1.25 times the untuned call lies between the two)."""
+    base, q = H.gaussian(10_000, 700, 128, 42)
+    data = build_index(base, ef_construction=100)
+    tuned, untuned = H.HnswIndex.from_bytes(data), H.HnswIndex.from_bytes(data)
+    want = O.Index(data).search(q[:1], 10, 256)
+    best, trials = tuned.autotune(q[:sample], 10, 256, reps=3)
+    if sample == 1:  # the heuristic's trial takes a team, the others a warp
+        assert best["heuristic"]
+        assert best["ms"] < 0.8 * min(t["ms"] for t in trials if not t["heuristic"])
+    times = {tuned: [], untuned: []}
+    for _ in range(40):
+        for ix in times:
+            t = time.perf_counter()
+            got = ix.search_arrays(q[:1], 10, 256, mode=H.MODE_AUTO)
+            times[ix].append(time.perf_counter() - t)
+            assert_same(got, want, "tuned" if ix is tuned else "untuned")
+    assert statistics.median(times[tuned]) < 1.25 * statistics.median(times[untuned])
