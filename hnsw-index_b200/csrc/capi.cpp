@@ -179,7 +179,8 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
                           const uint32_t* d_ks, const uint32_t* d_efs, const uint64_t* d_fbits, const uint8_t* d_fused,
                           const uint32_t* d_fids,
                           uint64_t* d_keys, float* d_dist, uint32_t* d_count, int32_t* d_status, uint32_t ef_max,
-                          uint32_t out_stride, cudaStream_t stream, const SearchGeometry* force, bool publish) {
+                          uint32_t out_stride, cudaStream_t stream, const SearchGeometry* force, bool publish,
+                          bool reserve) {
     hnsw_search_opts o = o_in;
     if (o.mode != HNSW_MODE_PLAIN && o.mode != HNSW_MODE_PERSISTENT && o.mode != HNSW_MODE_AUTO)
         return set_error(HNSW_ERR_INVALID_ARGUMENT, "unknown search mode");
@@ -246,7 +247,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     CU(s->work.ensure(32), "cudaMalloc work counters");
     CU(s->overflow.ensure(std::max<size_t>(nq, 1) * 4), "cudaMalloc overflow list");
     CU(s->overflow2.ensure(std::max<size_t>(nq, 1) * 4), "cudaMalloc overflow list");
-    CU(cudaMemsetAsync(s->work.p, 0, 32, stream), "memset work counters");
+    if (!reserve) CU(cudaMemsetAsync(s->work.p, 0, 32, stream), "memset work counters");
     SearchArgs a;
     a.ix = gi->view;
     a.queries = d_q;
@@ -315,8 +316,23 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     // warp kernels.
     const uint32_t bit_words = ((gi->view.n + 31) / 32 + 3) & ~3u;
     if (team.blocks || redo.blocks) {
-        auto far = [](const TeamGeometry& g) { return size_t(g.blocks) * g.far_cap * 8; };
-        auto bits = [&](const TeamGeometry& g) { return g.bitmap_words ? 0 : size_t(g.blocks) * bit_words * 4; };
+        // Sizes follow the batch's team count rounded up to a power of two, so
+        // that calls of rising size grow them a few times only: growing frees
+        // the old buffer, which waits for all work on the device.
+        auto pow2 = [](size_t x) {
+            size_t p = 1;
+            while (p < x) p <<= 1;
+            return p;
+        };
+        auto far = [&](const TeamGeometry& g) {
+            const size_t need = size_t(g.blocks) * g.far_cap * 8;
+            return g.blocks ? std::max(need, std::min(pow2(need), size_t(1) << 28)) : size_t(0);
+        };
+        auto bits = [&](const TeamGeometry& g) {
+            if (g.bitmap_words || !g.blocks) return size_t(0);
+            const size_t rows = std::max<size_t>(g.blocks, std::min(pow2(g.blocks), size_t(gi->num_sms) * 2));
+            return rows * bit_words * 4;
+        };
         cudaError_t e = s->team_far.ensure(std::max(far(team), far(redo)));
         if (e == cudaSuccess) e = s->team_bits.ensure(std::max(bits(team), bits(redo)));
         if (e != cudaSuccess) {
@@ -352,9 +368,10 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         CU(s->order.ensure(nq * 5), "cudaMalloc query order");
         const uint32_t slots = a.persistent && warp_route ? a.spill_slots : uint32_t(gi->num_sms) * 16;
         uint32_t* route = s->work.as<uint32_t>() + 5;
-        CU(launch_query_order(a, s->order.as<uint32_t>(), s->order.as<uint8_t>() + nq * 4, slots, team.blocks, route,
-                              stream),
-           "query order");
+        if (!reserve)
+            CU(launch_query_order(a, s->order.as<uint32_t>(), s->order.as<uint8_t>() + nq * 4, slots, team.blocks,
+                                  route, stream),
+               "query order");
         a.order = s->order.as<uint32_t>();
         if (warp_route) a.route = route;
     }
@@ -393,6 +410,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         for (size_t i = 0; i < ids.size(); ++i) ids[i] = uint32_t(i);
         CU(cudaMemcpy(s->last_tab.p, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice), "copy last-resort table");
     }
+    if (reserve) return HNSW_OK;
     a.overflow_list2 = s->overflow2.as<uint32_t>();
     a.overflow_count2 = s->work.as<uint32_t>() + 4;
     if (plans) {
@@ -431,6 +449,30 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     last.cold_slots = kLastResortWarps;
     last.cold_private = 1;
     CU(launch_search_retry(last, kLastResortWarps, stream), "search last-resort kernel");
+    return HNSW_OK;
+}
+
+// Grows the slot's buffers to what batches of up to max_nq queries with a k
+// and an ef per query need, so that none of them allocates (growing a buffer
+// frees the old one, which waits for the batches of every other slot). The
+// schedule differs by ef bucket, and its smaller ones can need more memory
+// (more warps resident), so each is gone through: about 1 ms a slot.
+int hnswgpu::reserve_search(hnsw_gpu_index* gi, Slot* s, uint32_t max_nq, uint32_t max_ef, const hnsw_search_opts& o,
+                            bool filtered) {
+    // Only whether these are given is looked at.
+    const uint32_t* given = reinterpret_cast<const uint32_t*>(s);
+    for (uint32_t nq : {max_nq, std::min<uint32_t>(max_nq, 2 * uint32_t(gi->num_sms))})
+        for (bool f : {false, true}) {
+            if (f && !filtered) continue;
+            for (uint32_t ef = std::min<uint32_t>(1056, max_ef);; ef -= 32) {
+                const uint32_t ef_max = ef > 1024 ? max_ef : ef;
+                int r = enqueue_search(gi, s, nullptr, nq, o, given, given,
+                                       f ? reinterpret_cast<const uint64_t*>(given) : nullptr, nullptr, nullptr, nullptr,
+                                       nullptr, nullptr, nullptr, ef_max, o.out_stride, s->stream, nullptr, true, true);
+                if (r != HNSW_OK) return r;
+                if (ef <= 32) break;
+            }
+        }
     return HNSW_OK;
 }
 

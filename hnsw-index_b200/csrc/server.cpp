@@ -101,6 +101,40 @@ struct hnsw_gpu_server {
 
 namespace {
 
+hnsw_search_opts server_opts(const hnsw_gpu_server* s) {
+    hnsw_search_opts o{};
+    o.k = s->cfg.max_k;
+    o.ef = s->cfg.max_ef;
+    o.quantized = s->cfg.quantized;
+    o.filter_nbits = s->cfg.filter_nbits;
+    o.filter_by_node = s->cfg.filter_by_node;
+    o.filter_stride = s->words;
+    o.out_stride = s->cfg.max_k;
+    o.mode = s->cfg.mode;
+    return o;
+}
+
+// Allocates what a batch slot's launches will need, before the first: growth
+// later on would wait for every batch in flight while requests queue. On
+// failure, and past `budget` bytes in all, slots are left to grow as they go.
+void reserve_slot(hnsw_gpu_server* s, Slot* sl, size_t* budget) {
+    size_t before = 0, after = 0, total = 0;
+    if (*budget == 0 || cudaMemGetInfo(&before, &total) != cudaSuccess) return;
+    const size_t B = s->cfg.max_batch;
+    bool ok = sl->q.ensure(B * s->dim * 4) == cudaSuccess && sl->ks.ensure(B * 4) == cudaSuccess &&
+              sl->efs.ensure(B * 4) == cudaSuccess;
+    if (ok && s->cfg.filter_count)
+        ok = sl->fused.ensure(B) == cudaSuccess && sl->fids.ensure(B * 4) == cudaSuccess;
+    ok = ok && reserve_search(s->index, sl, s->cfg.max_batch, std::max(s->cfg.max_k, s->cfg.max_ef), server_opts(s),
+                              s->cfg.filter_count != 0) == HNSW_OK;
+    if (!ok || cudaMemGetInfo(&after, &total) != cudaSuccess) {
+        cudaGetLastError();
+        *budget = 0;
+        return;
+    }
+    *budget -= std::min(*budget, before > after ? before - after : 0);
+}
+
 int stage_and_launch(hnsw_gpu_server* s, BatchSlot& b, std::vector<uint64_t>& tickets) {
     TraceRange trace("hnsw.server_batch");
     const uint32_t n = uint32_t(tickets.size());
@@ -138,15 +172,7 @@ int stage_and_launch(hnsw_gpu_server* s, BatchSlot& b, std::vector<uint64_t>& ti
         d_fu = sl->fused.as<uint8_t>();
         d_fi = sl->fids.as<uint32_t>();
     }
-    hnsw_search_opts o{};
-    o.k = K;
-    o.ef = s->cfg.max_ef;
-    o.quantized = s->cfg.quantized;
-    o.filter_nbits = s->cfg.filter_nbits;
-    o.filter_by_node = s->cfg.filter_by_node;
-    o.filter_stride = s->words;
-    o.out_stride = K;
-    o.mode = s->cfg.mode;
+    const hnsw_search_opts o = server_opts(s);
     b.finished.assign(n, 0);
     b.remaining = n;
     // Scratch sized for the batch's own largest max(ef, k).
@@ -334,6 +360,11 @@ int hnsw_gpu_server_start(hnsw_gpu_index* index, const hnsw_server_config* cfg_i
         CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&b.d_count), b.h_count, 0), "mapped counts");
         CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&b.d_status), b.h_status, 0), "mapped statuses");
     }
+    // Half of the memory that is free now, at most.
+    size_t budget = 0, total = 0;
+    if (cudaMemGetInfo(&budget, &total) != cudaSuccess) cudaGetLastError();
+    budget /= 2;
+    for (BatchSlot& b : s->batches) reserve_slot(s.get(), b.slot, &budget);
     hnsw_gpu_server* raw = s.get();
     raw->dispatcher = std::thread(dispatch_loop, raw);
     *out = s.release();

@@ -244,7 +244,11 @@ int hnsw_gpu_read_counters(hnsw_gpu_index* index, uint32_t* host_out, size_t nq)
  * thread batches pending requests and launches each batch on its own stream
  * as soon as one of max_inflight device scratch slots is free, so requests
  * arriving while earlier batches run join the next launch and overlap on the
- * device. Each result equals the same search run alone. */
+ * device. Each result equals the same search run alone. The start allocates
+ * every slot's device scratch for max_batch, max_k and max_ef (6.3 GB a slot
+ * at 10M x 128 with filters, most of it one bit per node for each resident
+ * warp), at most half of the free memory in all; slots past that grow as they
+ * go, and the index keeps the scratch after the stop. */
 
 typedef struct hnsw_gpu_server hnsw_gpu_server;
 

@@ -155,3 +155,33 @@ def test_cancelled_requests_report_cancelled_and_others_stand(served):
     for i, (keys, _, status, _) in enumerate(after):
         assert status == 0
         np.testing.assert_array_equal(keys, ref[0][i, :int(ref[2][i])])
+
+
+def test_batches_of_rising_size_allocate_nothing(served):
+    """The slots' buffers are there when the server starts: requests that
+    arrive one by one, then in small and in full batches, with every ef and
+    with filters, leave the device's free memory as it was (the far lists of a
+    slot alone would take 45 MiB more)."""
+    import torch
+
+    base, queries, data = served
+    nbits = 20000
+    q = np.tile(queries, (4, 1))
+    ks, efs, fids, bank = make_requests(q, nbits, 5)
+    efs[::7] = 32  # buckets of their own
+    free = []
+    for _ in range(2):  # the first round loads the kernels
+        gi = H.HnswIndex.from_bytes(data)
+        srv = H.Server(gi, max_batch=1024, max_inflight=2, max_pending=1 << 14, max_k=100, max_ef=512, linger_us=50,
+                       filter_nbits=nbits, filter_bank=bank)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info(0)[0])
+        for n, gap in ((20, 3000.0), (600, 5.0), (2400, 0.0), (2400, 0.2)):
+            arrivals = np.arange(n) * gap
+            st = srv.replay(q[:n], arrivals, ks[:n], efs[:n], fids[:n])[3]
+            assert (st == 0).all()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info(0)[0])
+        srv.stop()
+        gi.close()
+    assert free[2] - free[3] <= 4 << 20
