@@ -301,14 +301,19 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     if (teams && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
     bool warp_route = !team.blocks || !small;
-    // Queries that outgrow a warp's scratch are redone by teams (one per SM):
-    // a warp of the retry kernel takes milliseconds for one, and the batch
-    // waits for it.
+    // Queries that outgrow a warp's scratch are redone by teams: a warp of the
+    // retry kernel takes milliseconds for one, and the batch waits for it. One
+    // team per SM (its visited bitmap stays in shared memory up to 1.4 M nodes)
+    // for persistent warps, which continue such queries in their spill areas
+    // and leave few; as many as fit for plain warps, which leave every query
+    // that outgrows the visited hash (50,000 filtered int8 queries on 5M x 96:
+    // a call takes 2.53 s with one team per SM, 2.08 s with 592 retry warps
+    // and 1.39 s with two teams per SM, 90 ms of it in the warp kernel).
     TeamGeometry redo;
     if (redo_teams && !o.traversal && tags == 0 && warp_route && ef_max <= 1024) {
-        SearchArgs one = a;
-        one.nq = uint32_t(gi->num_sms);
-        CU(plan_search_team(one, ef_max, gi->num_sms, &redo), "team occupancy");
+        SearchArgs all = a;
+        all.nq = uint32_t(gi->num_sms) * (persistent ? 1 : 2);
+        CU(plan_search_team(all, ef_max, gi->num_sms, &redo), "team occupancy");
     }
     // Both launches share the team buffers: each buffer grows once, to what
     // the larger needs (growing it for one after the other would free what the

@@ -79,6 +79,26 @@ def test_team_retry_of_queries_that_outgrow_a_warp(ef):
     assert_same(got, oi.search(q, 10, ef), f"ef={ef}")
 
 
+@pytest.mark.parametrize("quantized", [False, True])
+def test_plain_filtered_batch_that_is_mostly_redone(quantized):
+    """Plain warps hand every query that outgrows the visited hash (2048 slots
+    at ef = 32) to the teams' retry pass: here more than teams are resident."""
+    n, nq = 30000, 900
+    base, q = H.mixture(n, nq, 24, 30, 0.4, 5)
+    data = build_index(base, metric=1, ef_construction=60, quantize=True)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    rng = np.random.default_rng(8)
+    words = (n + 63) // 64
+    bank = np.stack([H.key_bitmap(np.nonzero(rng.random(n) < p)[0].astype(np.uint64), n) for p in (0.01, 0.02, 0.9)])
+    ids = rng.integers(0, 3, nq).astype(np.uint32)
+    kw = dict(filter_bits=bank, filter_nbits=n, filter_stride=words, filter_ids=ids, quantized=quantized, mode=0)
+    gi.set_counters(True)
+    got = gi.search_arrays(q, 10, 32, **kw)
+    assert (gi.read_counters(nq)[:, 0] > 2048).sum() > 400
+    ref = oi.search(q, 10, 32, filter_bits=bank[ids], filter_nbits=n, filter_stride=words, quantized=quantized)
+    assert_same(got, ref, f"quantized={quantized}")
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("sel", [0.02, 0.9])
 def test_batches_routed_on_the_device(mode, sel):
