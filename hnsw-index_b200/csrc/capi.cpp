@@ -369,9 +369,10 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         a.spill_slots = warps;
     }
     if (!warp_route) geo.cold = 0;
-    if (team.blocks && varied && nq > team.blocks) {
+    if (team.blocks && varied && (warp_route || nq > team.blocks)) {
         CU(s->order.ensure(nq * 5), "cudaMalloc query order");
-        const uint32_t slots = a.persistent && warp_route ? a.spill_slots : uint32_t(gi->num_sms) * 16;
+        uint32_t slots = std::max<uint32_t>(a.spill_slots, 1);  // warps resident at once
+        if (!a.persistent && warp_route) CU(resident_search_warps(a, geo, gi->num_sms, &slots), "occupancy");
         uint32_t* route = s->work.as<uint32_t>() + 5;
         if (!reserve)
             CU(launch_query_order(a, s->order.as<uint32_t>(), s->order.as<uint8_t>() + nq * 4, slots, team.blocks,

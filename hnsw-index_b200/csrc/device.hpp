@@ -183,6 +183,9 @@ __host__ __device__ inline uint32_t tc_query_bytes(const SearchArgs& a) {
     return a.traversal ? a.ix.dt * 2u * (a.traversal == 2 ? 2u : 1u) : 0u;
 }
 
+// Warps resident at once of the kernel that launch_search takes for the batch.
+cudaError_t resident_search_warps(const SearchArgs& args, const SearchGeometry& geo, int num_sms, uint32_t* warps);
+
 constexpr uint32_t kLastResortWarps = 4;
 
 // Team traversal (search_team.cu): a block of warps per query. blocks == 0:

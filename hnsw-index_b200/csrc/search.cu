@@ -161,6 +161,19 @@ cudaError_t persistent_warps(const SearchGeometry& g_in, uint32_t dp, uint32_t d
     return cudaSuccess;
 }
 
+cudaError_t resident_search_warps(const SearchArgs& args, const SearchGeometry& geo_in, int num_sms, uint32_t* warps) {
+    SearchGeometry geo = geo_in;
+    geo.bytes_per_warp = geometry_bytes_per_warp(geo, args.ix.dp, args.ix.dc);
+    const SearchKernel kern = pick_search_kernel(args, geo, num_sms);
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kern));
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, int(32 * geo.warps_per_block),
+                                                      size_t(geo.bytes_per_warp) * geo.warps_per_block);
+    *warps = uint32_t(std::max(per_sm, 1)) * geo.warps_per_block * uint32_t(num_sms);
+    return e;
+}
+
 cudaError_t launch_search_retry(const SearchArgs& args, uint32_t warps, cudaStream_t stream) {
     const uint32_t wpb = 4;
     const size_t smem =

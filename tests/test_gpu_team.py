@@ -115,6 +115,18 @@ def test_batches_routed_on_the_device(mode, sel):
     assert_same(gi.search_arrays(q, 10, 16, mode=mode, **kw), oi.search(q, 10, 16, **kw), f"mode={mode} sel={sel}")
 
 
+@pytest.mark.parametrize("nq,ef", [(400, 900), (900, 1024), (900, 1100)])
+def test_plain_batches_of_few_resident_warps(nq, ef):
+    """At ef near 1024 a plain warp's scratch leaves four warps per SM or
+    fewer, which the route compares with two teams; above it no team fits."""
+    n = 5000
+    base, q = H.mixture(n, nq, 24, 30, 0.4, 5)
+    data = build_index(base, metric=1, ef_construction=60)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    efs = np.random.default_rng(3).integers(ef - 200, ef + 1, nq).astype(np.uint32)
+    assert_same(gi.search_arrays(q, 10, 16, mode=0, efs=efs), oi.search(q, 10, 16, efs=efs), f"nq={nq} ef={ef}")
+
+
 def test_team_with_its_visited_bitmap_in_global_memory():
     n = 800_000
     base, q = H.mixture(n, 160, 4, 500, 0.3, 2)
