@@ -294,13 +294,23 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     // A team of warps per query where one warp each would leave the batch
     // waiting on memory latency: up to two teams per SM, or four when the
     // queries are alike. Larger batches of unlike queries (filters, an ef per
-    // query) are decided on the device from their expected work.
+    // query) are decided on the device from their expected work, those whose
+    // queries share one filter and one ef by the same rule here: their expected
+    // work is equal, and ordering them would only cost the order kernel's time.
     TeamGeometry team;
     const bool plans = o.exact_below > 0.0f && d_fbits, varied = d_efs || d_fbits;
     const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
     if (teams && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
     bool warp_route = !team.blocks || !small;
+    const bool equal_work = !d_efs && !d_ks && (!d_fbits || (!o.filter_stride && !d_fused));
+    if (team.blocks && !small && equal_work) {
+        uint32_t warps = 0;
+        CU(resident_search_warps(a, geo, gi->num_sms, &warps), "occupancy");
+        const float q = float(nq);
+        warp_route = kTeamSpeed * std::max(1.0f, q / float(warps)) <= std::max(1.0f, q / float(team.blocks));
+        if (warp_route) team = TeamGeometry();
+    }
     // Queries that outgrow a warp's scratch are redone by teams: a warp of the
     // retry kernel takes milliseconds for one, and the batch waits for it. One
     // team per SM (its visited bitmap stays in shared memory up to 1.4 M nodes)
@@ -369,7 +379,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         a.spill_slots = warps;
     }
     if (!warp_route) geo.cold = 0;
-    if (team.blocks && varied && (warp_route || nq > team.blocks)) {
+    if (team.blocks && varied && !equal_work && (warp_route || nq > team.blocks)) {
         CU(s->order.ensure(nq * 5), "cudaMalloc query order");
         uint32_t slots = std::max<uint32_t>(a.spill_slots, 1);  // warps resident at once
         if (!a.persistent && warp_route) CU(resident_search_warps(a, geo, gi->num_sms, &slots), "occupancy");

@@ -205,6 +205,8 @@ cudaError_t launch_search_team(const SearchArgs& args, const TeamGeometry& geo, 
 // the batch (kRoute*) given the warps or teams resident at once; `bucket` is
 // scratch (nq bytes).
 constexpr uint32_t kRouteWarp = 1, kRouteTeam = 2;
+// A team's speed in warps (the comment at query_order_kernel has the figures).
+constexpr float kTeamSpeed = 2.2f;
 cudaError_t launch_query_order(const SearchArgs& args, uint32_t* order, uint8_t* bucket, uint32_t warp_slots,
                                uint32_t team_slots, uint32_t* route, cudaStream_t stream);
 

@@ -988,7 +988,6 @@ __device__ __forceinline__ float expected_work(const SearchArgs& a, uint32_t qi)
 __global__ void __launch_bounds__(1024) query_order_kernel(SearchArgs a, uint32_t* order, uint8_t* bucket,
                                                            float warp_slots, float team_slots, uint32_t* route) {
     constexpr uint32_t B = 128;
-    constexpr float kTeamSpeed = 2.2f;
     __shared__ uint32_t hist[B], next[B];
     __shared__ float wsum[32], wmax[32];
     for (uint32_t i = threadIdx.x; i < B; i += blockDim.x) hist[i] = 0;

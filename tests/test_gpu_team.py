@@ -115,6 +115,21 @@ def test_batches_routed_on_the_device(mode, sel):
     assert_same(gi.search_arrays(q, 10, 16, mode=mode, **kw), oi.search(q, 10, 16, **kw), f"mode={mode} sel={sel}")
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("nq", [297, 640, 700, 1500])
+def test_batches_of_one_filter(nq, mode):
+    """One filter and one ef for the batch: teams up to about 650 queries,
+    one warp per query above."""
+    n = 6000
+    base, q = H.mixture(n, nq, 24, 30, 0.4, 5)
+    data = build_index(base, ef_construction=60, quantize=True)
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    for sel in (0.01, 0.9):
+        bits = H.key_bitmap(np.nonzero(np.random.default_rng(8).random(n) < sel)[0].astype(np.uint64), n)
+        kw = dict(filter_bits=bits, filter_nbits=n, quantized=sel > 0.5)
+        assert_same(gi.search_arrays(q, 10, 48, mode=mode, **kw), oi.search(q, 10, 48, **kw), f"nq={nq} sel={sel}")
+
+
 @pytest.mark.parametrize("nq,ef", [(400, 900), (900, 1024), (900, 1100)])
 def test_plain_batches_of_few_resident_warps(nq, ef):
     """At ef near 1024 a plain warp's scratch leaves four warps per SM or
