@@ -1537,10 +1537,16 @@ __device__ __forceinline__ void search_body(const SearchArgs& a, const SearchGeo
         if (V == 1) attach_cold(w, a, slot, a.cold_next);
         for (;;) {
             uint32_t qi = 0;
-            if (lane == 0) qi = atomicAdd(a.work_next, 1u);
+            // One lane looks the query up: with all 32 reading the order, the
+            // variant for filtered batches came out 10 % slower (1,000 queries
+            // through a 20 % filter on 100k x 96: 2.13 ms, so 1.92; 10,000:
+            // 12.7 and 11.5), though its loop is the same source.
+            if (lane == 0) {
+                qi = atomicAdd(a.work_next, 1u);
+                if (a.order && qi < a.nq) qi = a.order[qi];
+            }
             qi = __shfl_sync(kFull, qi, 0);
             if (qi >= a.nq) break;
-            if (a.order) qi = __ldg(a.order + qi);
             const int32_t st = run_query<V, DK>(a, w, qi, qi);
             end_spill(w);
             if (st == ST_OVERFLOW && lane == 0) {
