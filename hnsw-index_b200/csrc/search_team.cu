@@ -955,8 +955,9 @@ __global__ void __launch_bounds__(512, 1) search_team_kernel(SearchArgs a, TeamG
 }
 
 // Expected expansions of a query: a filtered walk goes on until ef admitted
-// nodes are found, i.e. about ef / selectivity, the selectivity taken from 32
-// words of the bitmap (the index's size at most).
+// nodes are found, i.e. about ef / selectivity (the index's size at most). The
+// selectivity is that of 32 words spread over the nodes where bits are indexed
+// by node, else of 256 nodes' keys: keys need not lie in [0, n).
 __device__ __forceinline__ float expected_work(const SearchArgs& a, uint32_t qi) {
     const DeviceIndexView& ix = a.ix;
     const uint32_t k = min(a.ks ? a.ks[qi] : a.k, a.out_stride);
@@ -964,12 +965,24 @@ __device__ __forceinline__ float expected_work(const SearchArgs& a, uint32_t qi)
     if (a.filter_bits != nullptr && (a.filter_used == nullptr || a.filter_used[qi] != 0)) {
         const size_t fsel = a.filter_ids ? size_t(a.filter_ids[qi]) : size_t(qi);
         const uint64_t* bits = a.filter_bits + (a.filter_stride ? fsel * a.filter_stride : 0);
-        const uint32_t nwords = uint32_t(min(a.filter_nbits, uint64_t(ix.n)) >> 6);
-        const uint32_t m = min(nwords, 32u);
-        uint32_t set = 0;
-        for (uint32_t i = 0; i < m; ++i)
-            set += uint32_t(__popcll(static_cast<long long>(__ldg(bits + uint64_t(nwords) * i / m))));
-        cost = cost * float(64u * max(m, 1u)) / float(max(set, 1u));
+        uint32_t set = 0, of = 0;
+        if (ix.keys_are_ids || a.filter_by_node) {
+            const uint32_t nwords = max(ix.n >> 6, 1u), m = min(nwords, 32u);
+            of = 64u * m;
+#pragma unroll 8
+            for (uint32_t i = 0; i < m; ++i) {
+                const uint64_t w = nwords > 32u ? (uint64_t(nwords) * i) >> 5 : i;
+                if (w * 64 < a.filter_nbits) set += uint32_t(__popcll(static_cast<long long>(__ldg(bits + w))));
+            }
+        } else {
+            of = min(ix.n, 256u);
+#pragma unroll 8
+            for (uint32_t i = 0; i < of; ++i) {
+                const uint64_t key = __ldg(ix.keys + (ix.n > 256u ? (uint64_t(ix.n) * i) >> 8 : i));
+                if (key < a.filter_nbits) set += uint32_t(__ldg(bits + (key >> 6)) >> (key & 63)) & 1u;
+            }
+        }
+        cost = cost * float(max(of, 1u)) / float(max(set, 1u));
     }
     return fminf(fmaxf(cost, 1.0f), float(max(ix.live, 1u)));
 }

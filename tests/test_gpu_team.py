@@ -115,6 +115,33 @@ def test_batches_routed_on_the_device(mode, sel):
     assert_same(gi.search_arrays(q, 10, 16, mode=mode, **kw), oi.search(q, 10, 16, **kw), f"mode={mode} sel={sel}")
 
 
+def test_sparse_keys_are_routed_like_dense_ones():
+    """Keys far above the node count, one query in a hundred with a filter of
+    90 %: the expected work is that of the same queries on dense keys. (Read
+    below the node count the bitmap is empty, those queries seem to scan the
+    index, and the batch goes to teams: 1.37 times the time; 1.04 now.)"""
+    n, nq, first = 20000, 12000, 1 << 20
+    base, q = H.mixture(n, nq, 32, 40, 0.4, 5)
+    admitted = np.nonzero(np.random.default_rng(8).random(n) < 0.9)[0].astype(np.uint64)
+    used = (np.arange(nq) % 100 == 0).astype(np.uint8)
+    data = [build_index(base, ef_construction=60, keys=np.arange(n, dtype=np.uint64) + off, parallel=False)
+            for off in (0, first)]
+    calls, times = [], [[], []]
+    for d, off in zip(data, (0, first)):
+        gi = H.HnswIndex.from_bytes(d)
+        kw = dict(filter_bits=H.key_bitmap(admitted + np.uint64(off), n + off), filter_nbits=n + off)
+        calls.append((gi, dict(kw, filter_used=used)))
+        kw["filter_used"] = used[:900]
+        assert_same(gi.search_arrays(q[:900], 10, 64, **kw), O.Index(d).search(q[:900], 10, 64, **kw), f"from {off}")
+    for _ in range(15):
+        for (gi, kw), ts in zip(calls, times):
+            t = time.perf_counter()
+            got = gi.search_arrays(q, 10, 64, mode=1, **kw)
+            ts.append(time.perf_counter() - t)
+            assert (got[3] == 0).all()
+    assert statistics.median(times[1]) < 1.2 * statistics.median(times[0])
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("nq", [297, 640, 700, 1500])
 def test_batches_of_one_filter(nq, mode):
