@@ -325,6 +325,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         all.nq = uint32_t(gi->num_sms) * (persistent ? 1 : 2);
         CU(plan_search_team(all, ef_max, gi->num_sms, &redo), "team occupancy");
     }
+    auto ordered = [&] { return team.blocks && varied && !equal_work && (warp_route || nq > team.blocks); };
     // Both launches share the team buffers: each buffer grows once, to what
     // the larger needs (growing it for one after the other would free what the
     // first was planned with). Without memory for them the batch takes the
@@ -350,6 +351,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         };
         cudaError_t e = s->team_far.ensure(std::max(far(team), far(redo)));
         if (e == cudaSuccess) e = s->team_bits.ensure(std::max(bits(team), bits(redo)));
+        if (e == cudaSuccess && ordered()) e = s->order.ensure(nq * 5);
         if (e != cudaSuccess) {
             cudaGetLastError();
             team = redo = TeamGeometry();
@@ -379,8 +381,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         a.spill_slots = warps;
     }
     if (!warp_route) geo.cold = 0;
-    if (team.blocks && varied && !equal_work && (warp_route || nq > team.blocks)) {
-        CU(s->order.ensure(nq * 5), "cudaMalloc query order");
+    if (ordered()) {
         uint32_t slots = std::max<uint32_t>(a.spill_slots, 1);  // warps resident at once
         if (!a.persistent && warp_route) CU(resident_search_warps(a, geo, gi->num_sms, &slots), "occupancy");
         uint32_t* route = s->work.as<uint32_t>() + 5;

@@ -98,11 +98,13 @@ def test_allocation_failure_at_open_leaves_nothing_behind():
     assert gi.len() == 2000
 
 
-def test_team_buffers_that_cannot_grow_leave_the_batch_to_the_warp_kernels():
+@pytest.mark.parametrize("first", [1, 296])
+def test_team_buffers_that_cannot_grow_leave_the_batch_to_the_warp_kernels(first):
     """A batch that may take teams and whose overflowing queries are redone by
-    teams plans both on one far list. Above 226,719 nodes the second needs a
-    little more than the first, so after a batch that allocated the first's
-    size exactly the buffer has to grow; when that fails neither may run."""
+    teams plans both on the same buffers. After a batch that allocated what
+    fewer teams need (first = 1) the far list has to grow, after one of 296
+    queries only the query order; when that fails the warp kernels take the
+    batch, with the old buffer gone."""
     n, nq = 240_000, 900
     base, q = H.mixture(n, nq, 4, 300, 0.3, 2)
     b = H.IndexBuilder(4, H.Metric.L2, H.HnswParams(m=4, ef_construction=16, seed=7))
@@ -114,7 +116,7 @@ def test_team_buffers_that_cannot_grow_leave_the_batch_to_the_warp_kernels():
     gi.set_schedule(ef_cap=64, hash_cap=2048, warps_per_block=2)  # every buffer but the teams'
     _same(gi.search_arrays(q, 10, 16, efs=efs), ref)
     gi.set_schedule()
-    _same(gi.search_arrays(q[:296], 10, 16, efs=efs[:296]), tuple(x[:296] for x in ref))
+    _same(gi.search_arrays(q[:first], 10, 16, efs=efs[:first]), tuple(x[:first] for x in ref))
     try:
         H.debug_fail_allocations(1)
         _same(gi.search_arrays(q, 10, 16, efs=efs), ref)
