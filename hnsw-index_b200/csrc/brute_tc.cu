@@ -222,12 +222,17 @@ struct TileNorms {
     }
 };
 
+// The i-th row tile of a launch.
+__device__ __forceinline__ uint32_t row_tile(const TcScoreArgs& a, uint32_t i) {
+    return a.spread ? uint32_t(uint64_t(i) * a.spread / a.n_tiles) : i;
+}
+
 // Dense epilogue (threshold sample pass): this lane's query q against the
 // 256 rows row_base .. row_base + 255 held in TMEM columns taddr .. taddr +
-// 255 of its lane; every distance of the sample's row range is written,
+// 255 of its lane; every distance is written, at `pos` of the query's sample,
 // four at a time (+inf past the last row). All 32 lanes call.
 __device__ __forceinline__ void epilogue_dense(const TcScoreArgs& a, uint32_t taddr, uint32_t q, uint32_t row_base,
-                                               const float* xn) {
+                                               uint32_t pos, const float* xn) {
     const bool qvalid = q < a.nq;
     const float qn = (qvalid && a.qnorm2) ? a.qnorm2[q] : 0.0f;
     const EpiConsts e{a.metric, a.n, xn};
@@ -236,10 +241,8 @@ __device__ __forceinline__ void epilogue_dense(const TcScoreArgs& a, uint32_t ta
         __syncwarp();
         tmem_ld32(taddr + c * 32, v);
         const uint32_t row0 = row_base + c * 32;
-        // The sample range starts at a.row0 (a multiple of 256) and holds a.ld
-        // (a multiple of 256) rows, so a chunk lies wholly inside or outside.
-        if (!qvalid || row0 < a.row0 || row0 >= a.row0 + a.ld) continue;
-        float4* out = reinterpret_cast<float4*>(a.dense + size_t(q) * a.ld + (row0 - a.row0));
+        if (!qvalid) continue;
+        float4* out = reinterpret_cast<float4*>(a.dense + size_t(q) * a.ld + pos + c * 32);
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
             float d[4];
@@ -386,8 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t q_tiles = a.q_tiles;
-    const uint32_t n_tiles = a.n_tile_end - a.n_tile_begin;
-    const uint32_t total = q_tiles * n_tiles;
+    const uint32_t total = q_tiles * a.n_tiles;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -416,9 +418,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t t = blockIdx.x; ok && t < total; t += gridDim.x) {
-                const uint32_t nt = a.n_tile_begin + t / q_tiles, qt = t % q_tiles;
+                const uint32_t nt = row_tile(a, t / q_tiles), qt = t % q_tiles;
                 if (t + gridDim.x < total)
-                    prefetch_next_b(&tmB, nt, a.n_tile_begin + (t + gridDim.x) / q_tiles, a.k_chunks, kT, a.lo_col,
+                    prefetch_next_b(&tmB, nt, row_tile(a, (t + gridDim.x) / q_tiles), a.k_chunks, kT, a.lo_col,
                                     int(kTileN), 0, blockIdx.x);
                 for (uint32_t k = 0; k < a.k_chunks; ++k) {
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1u;
@@ -498,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         unsigned char* stage = stage_base + size_t(warp - 2) * kStageBytesPerWarp;
         uint32_t tile_it = 0;
         for (uint32_t t = blockIdx.x; t < total; t += gridDim.x, ++tile_it) {
-            const uint32_t nt = a.n_tile_begin + t / q_tiles, qt = t % q_tiles;
+            const uint32_t nt = row_tile(a, t / q_tiles), qt = t % q_tiles;
             const uint32_t b = tile_it & 1u, use = tile_it >> 1;
             const uint32_t q = qt * kTileM + lane_base + uint32_t(lane);
             // The query's threshold and norm load while the MMAs run.
@@ -517,7 +519,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (lane == 0) mbar_arrive(&acc_empty[b]);
             };
             if (a.dense) {
-                epilogue_dense(a, taddr, q, nt * kTileN, reinterpret_cast<const float*>(stage));
+                epilogue_dense(a, taddr, q, nt * kTileN, t / q_tiles * kTileN,
+                               reinterpret_cast<const float*>(stage));
                 release();
             } else {
                 epilogue_candidates(a, taddr, q, nt * kTileN, thr, qn, stage, release);
@@ -647,8 +650,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const bool leader = rank == 0;
     const uint32_t pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const uint32_t q_pairs = a.q_tiles >> 1;
-    const uint32_t n_tiles = a.n_tile_end - a.n_tile_begin;
-    const uint32_t total = q_pairs * n_tiles;
+    const uint32_t total = q_pairs * a.n_tiles;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -680,9 +682,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t t = pair; ok && t < total; t += npairs) {
-                const uint32_t nt = a.n_tile_begin + t / q_pairs, qp2 = t % q_pairs;
+                const uint32_t nt = row_tile(a, t / q_pairs), qp2 = t % q_pairs;
                 if (t + npairs < total)
-                    prefetch_next_b(&tmB, nt, a.n_tile_begin + (t + npairs) / q_pairs, a.k_chunks, kT, a.lo_col,
+                    prefetch_next_b(&tmB, nt, row_tile(a, (t + npairs) / q_pairs), a.k_chunks, kT, a.lo_col,
                                     int(kTileN), int(rank * kHalfN), pair);
                 for (uint32_t k = 0; k < a.k_chunks; ++k) {
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1u;
@@ -773,7 +775,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         unsigned char* stage = stage_base + size_t(warp - 2) * kStageBytesPerWarp;
         uint32_t tile_it = 0;
         for (uint32_t t = pair; t < total; t += npairs, ++tile_it) {
-            const uint32_t nt = a.n_tile_begin + t / q_pairs, qp2 = t % q_pairs;
+            const uint32_t nt = row_tile(a, t / q_pairs), qp2 = t % q_pairs;
             const uint32_t b = tile_it & 1u, use = tile_it >> 1;
             const uint32_t q = (2 * qp2 + rank) * kTileM + lane_base + uint32_t(lane);
             const float thr = (q < a.nq && a.thr) ? a.thr[q] : 0.0f;
@@ -794,7 +796,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
             };
             if (a.dense) {
-                epilogue_dense(a, taddr, q, nt * kTileN, reinterpret_cast<const float*>(stage));
+                epilogue_dense(a, taddr, q, nt * kTileN, t / q_pairs * kTileN,
+                               reinterpret_cast<const float*>(stage));
                 release();
             } else {
                 epilogue_candidates(a, taddr, q, nt * kTileN, thr, qn, stage, release);
@@ -1052,7 +1055,7 @@ cudaError_t tc_score(const __nv_bfloat16* A, uint32_t qp, const __nv_bfloat16* B
         auto kern2 = split ? tc::score_pair_kernel<true> : tc::score_pair_kernel<false>;
         cudaError_t e2 = raise_smem_limit(reinterpret_cast<const void*>(kern2));
         if (e2 != cudaSuccess) return e2;
-        const uint32_t total2 = (a.q_tiles / 2) * (a.n_tile_end - a.n_tile_begin);
+        const uint32_t total2 = (a.q_tiles / 2) * a.n_tiles;
         if (total2 == 0) return cudaSuccess;
         const uint32_t npairs = std::max<uint32_t>(1, std::min<uint32_t>(total2, uint32_t(num_sms) / 2));
         kern2<<<2 * npairs, tc::kThreads, smem2, stream>>>(ma, mb, a);
@@ -1064,7 +1067,7 @@ cudaError_t tc_score(const __nv_bfloat16* A, uint32_t qp, const __nv_bfloat16* B
     auto kern = split ? tc::score_kernel<true> : tc::score_kernel<false>;
     cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kern));
     if (e != cudaSuccess) return e;
-    const uint32_t total = a.q_tiles * (a.n_tile_end - a.n_tile_begin);
+    const uint32_t total = a.q_tiles * a.n_tiles;
     if (total == 0) return cudaSuccess;
     const uint32_t grid = std::min<uint32_t>(total, uint32_t(num_sms));
     kern<<<grid, tc::kThreads, smem, stream>>>(ma, mb, a);

@@ -8,20 +8,22 @@
 
 namespace hnswgpu {
 
-// Arguments of one scoring launch over row tiles [n_tile_begin, n_tile_end)
-// (256 rows each) for all query tiles (128 queries each).
+// Arguments of one scoring launch over n_tiles row tiles (256 rows each) for
+// all query tiles (128 queries each): the first n_tiles, or with `spread` that
+// many spaced evenly over the first `spread` tiles.
 struct TcScoreArgs {
     uint32_t q_tiles = 0, k_chunks = 0;   // set by tc_score
     int terms = 1;                        // 1: plain BF16; 3: split (operands [hi | lo])
     uint32_t lo_col = 0;                  // set by tc_score: first column of the lo half
-    uint32_t n_tile_begin = 0, n_tile_end = 0;
+    uint32_t n_tiles = 0, spread = 0;
     uint32_t nq = 0, n = 0;               // valid queries / rows
     int metric = 0;
     const float* qnorm2 = nullptr;        // per query |q|^2 (L2)
     const float* xnorm2 = nullptr;        // per row |x|^2 (L2)
-    // Dense mode: distances of rows [row0, row0 + ld) into dense[q * ld + row - row0].
+    // Dense mode: distances of the i-th scored tile's rows into
+    // dense[q * ld + 256 i ..] (ld = 256 n_tiles; +inf past the last row).
     float* dense = nullptr;
-    uint32_t row0 = 0, ld = 0;
+    uint32_t ld = 0;
     // Candidate mode: rows whose distance <= thr[q] are appended as
     // (f32 bits << 32 | row) to cand[q * cand_cap + slot], slot = cand_count[q]++.
     const float* thr = nullptr;

@@ -109,3 +109,22 @@ def test_paired_kernel_metrics_and_ragged_batches(metric):
     same(tcres, fp)
     same(again, fp)
     same(tcres, O.brute(metric, base, queries, 10))
+
+
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("metric,n", [(0, 131_072), (1, 100_003)])
+def test_tensor_rows_stored_cluster_by_cluster(metric, n, pairs):
+    """The threshold's sample spans the base: 64 clusters stored in order leave
+    each query far fewer candidates than the 13,000 to 17,000 that a sample of
+    the first rows (two clusters) does, and no query falls back to FP32."""
+    rng = np.random.default_rng(n)
+    centers = rng.standard_normal((64, 96)).astype(np.float32)
+    base = centers[np.sort(rng.integers(0, 64, n))] + 0.3 * rng.standard_normal((n, 96)).astype(np.float32)
+    q = centers[rng.integers(0, 64, 200)] + 0.3 * rng.standard_normal((200, 96)).astype(np.float32)
+    bf = H.BruteForceIndex(96, H.Metric(metric))
+    bf.insert_batch(np.arange(n, dtype=np.uint64), base)
+    bf.set_pairs(pairs)
+    for precision in (H.Precision.BF16, H.Precision.BF16X3):
+        tcres = bf.search_arrays(q, 10, precision)
+        assert bf.last_candidates_per_query() <= n / 16
+        same(tcres, bf.search_arrays(q, 10, H.Precision.FP32))
