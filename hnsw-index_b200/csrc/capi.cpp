@@ -810,8 +810,8 @@ struct StagedBatch {
     const uint32_t* fids = nullptr;
 };
 
-static int stage_batch(Slot* s, const float* queries, size_t nq, size_t dim, const hnsw_search_opts& o,
-                       uint32_t stride, StagedBatch* out) {
+static int stage_batch(hnsw_gpu_index* gi, Slot* s, const float* queries, size_t nq, size_t dim,
+                       const hnsw_search_opts& o, uint32_t stride, StagedBatch* out) {
     cudaStream_t st = s->stream;
     CU(s->q.ensure(nq * dim * 4), "cudaMalloc queries");
     CU(cudaMemcpyAsync(s->q.p, queries, nq * dim * 4, cudaMemcpyHostToDevice, st), "copy queries");
@@ -852,7 +852,7 @@ static int stage_batch(Slot* s, const float* queries, size_t nq, size_t dim, con
         }
     }
     CU(s->out.ensure(nq, stride), "cudaMalloc outputs");
-    if (o.ks || o.filter_bits) CU(s->out.clear(st), "clear outputs");
+    if (o.ks || o.filter_bits || stride > gi->view.live) CU(s->out.clear(st), "clear outputs");
     out->ks = d_ks;
     out->efs = d_efs;
     out->fbits = d_fb;
@@ -896,7 +896,7 @@ int hnsw_gpu_search_batch(hnsw_gpu_index* gi, const float* queries, size_t nq, s
     std::unique_ptr<Slot, std::function<void(Slot*)>> hold(s, [gi](Slot* p) { gi->slots.release(p); });
     cudaStream_t st = s->stream;
     StagedBatch sb;
-    r = stage_batch(s, queries, nq, dim, o, stride, &sb);
+    r = stage_batch(gi, s, queries, nq, dim, o, stride, &sb);
     if (r != HNSW_OK) return r;
     r = enqueue_search(gi, s, s->q.as<float>(), nq, o, sb.ks, sb.efs, sb.fbits, sb.fused, sb.fids,
                        s->out.keys(), s->out.dist(), s->out.count(), s->out.status(), ef_bound, stride, st);
@@ -936,7 +936,7 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
     std::unique_ptr<Slot, std::function<void(Slot*)>> hold(s, [gi](Slot* p) { gi->slots.release(p); });
     cudaStream_t st = s->stream;
     StagedBatch sb;
-    r = stage_batch(s, queries, nq, dim, o, stride, &sb);
+    r = stage_batch(gi, s, queries, nq, dim, o, stride, &sb);
     if (r != HNSW_OK) return r;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     CU(cudaEventCreate(&ev[0]), "cudaEventCreate");
@@ -1319,6 +1319,7 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     CU(b->qprep.ensure(size_t(qp) * b->dp * 4), "cudaMalloc qprep");
     // Beside the outputs: the candidate counts, and the error word after them.
     CU(b->out.ensure(nq, k, (size_t(qp) + 1) * 4), "cudaMalloc outputs");
+    if (k > b->n) CU(b->out.clear(st), "clear outputs");
     uint32_t* d_ccount = b->out.extra();
     uint32_t* d_err = d_ccount + qp;
     a.queries = b->q.as<float>();
@@ -1465,7 +1466,7 @@ static int brute_search_fp32(hnsw_gpu_brute* b, const float* queries, size_t nq,
     CU(b->minima.ensure(nq * kBruteMinima * 4), "cudaMalloc lane minima");
     a.minima = b->minima.as<uint32_t>();
     CU(b->out.ensure(nq, kk), "cudaMalloc outputs");
-    if (f && f->bits) CU(b->out.clear(st), "clear outputs");
+    if ((f && f->bits) || k > b->n) CU(b->out.clear(st), "clear outputs");
     a.queries = b->q.as<float>();
     a.qprep = b->qprep.as<float>();
     a.part = b->part.as<uint64_t>();

@@ -104,9 +104,10 @@ struct Outputs {
     }
     // The buffer holds what another call, of another shape, left there, so the
     // entries beyond a row's count are zeroed: on the device before a call
-    // that will leave many (a k per query, a filter), else in the caller's
-    // arrays (few or none: rows with k above the number of live nodes, failed
-    // queries; the scan of 10,000 counts takes about 3 us).
+    // that will leave many (a k per query, a filter, k above the number of
+    // rows; 1,000 queries for the best 1,000 of 300: 1.9 ms, 2.9 on the host),
+    // else in the caller's arrays (failed queries; the scan of 10,000 counts
+    // takes about 3 us).
     cudaError_t clear(cudaStream_t st) {
         cleared = true;
         return cudaMemsetAsync(dev.p, 0, rows * stride * 12, st);
