@@ -222,11 +222,6 @@ struct TileNorms {
     }
 };
 
-// The i-th row tile of a launch.
-__device__ __forceinline__ uint32_t row_tile(const TcScoreArgs& a, uint32_t i) {
-    return a.spread ? uint32_t(uint64_t(i) * a.spread / a.n_tiles) : i;
-}
-
 // Dense epilogue (threshold sample pass): this lane's query q against the
 // 256 rows row_base .. row_base + 255 held in TMEM columns taddr .. taddr +
 // 255 of its lane; every distance is written, at `pos` of the query's sample,
@@ -418,9 +413,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t t = blockIdx.x; ok && t < total; t += gridDim.x) {
-                const uint32_t nt = row_tile(a, t / q_tiles), qt = t % q_tiles;
+                const uint32_t nt = t / q_tiles * a.tile_step, qt = t % q_tiles;
                 if (t + gridDim.x < total)
-                    prefetch_next_b(&tmB, nt, row_tile(a, (t + gridDim.x) / q_tiles), a.k_chunks, kT, a.lo_col,
+                    prefetch_next_b(&tmB, nt, (t + gridDim.x) / q_tiles * a.tile_step, a.k_chunks, kT, a.lo_col,
                                     int(kTileN), 0, blockIdx.x);
                 for (uint32_t k = 0; k < a.k_chunks; ++k) {
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1u;
@@ -500,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         unsigned char* stage = stage_base + size_t(warp - 2) * kStageBytesPerWarp;
         uint32_t tile_it = 0;
         for (uint32_t t = blockIdx.x; t < total; t += gridDim.x, ++tile_it) {
-            const uint32_t nt = row_tile(a, t / q_tiles), qt = t % q_tiles;
+            const uint32_t nt = t / q_tiles * a.tile_step, qt = t % q_tiles;
             const uint32_t b = tile_it & 1u, use = tile_it >> 1;
             const uint32_t q = qt * kTileM + lane_base + uint32_t(lane);
             // The query's threshold and norm load while the MMAs run.
@@ -682,9 +677,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t t = pair; ok && t < total; t += npairs) {
-                const uint32_t nt = row_tile(a, t / q_pairs), qp2 = t % q_pairs;
+                const uint32_t nt = t / q_pairs * a.tile_step, qp2 = t % q_pairs;
                 if (t + npairs < total)
-                    prefetch_next_b(&tmB, nt, row_tile(a, (t + npairs) / q_pairs), a.k_chunks, kT, a.lo_col,
+                    prefetch_next_b(&tmB, nt, (t + npairs) / q_pairs * a.tile_step, a.k_chunks, kT, a.lo_col,
                                     int(kTileN), int(rank * kHalfN), pair);
                 for (uint32_t k = 0; k < a.k_chunks; ++k) {
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1u;
@@ -775,7 +770,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         unsigned char* stage = stage_base + size_t(warp - 2) * kStageBytesPerWarp;
         uint32_t tile_it = 0;
         for (uint32_t t = pair; t < total; t += npairs, ++tile_it) {
-            const uint32_t nt = row_tile(a, t / q_pairs), qp2 = t % q_pairs;
+            const uint32_t nt = t / q_pairs * a.tile_step, qp2 = t % q_pairs;
             const uint32_t b = tile_it & 1u, use = tile_it >> 1;
             const uint32_t q = (2 * qp2 + rank) * kTileM + lane_base + uint32_t(lane);
             const float thr = (q < a.nq && a.thr) ? a.thr[q] : 0.0f;

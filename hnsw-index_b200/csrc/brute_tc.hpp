@@ -8,14 +8,13 @@
 
 namespace hnswgpu {
 
-// Arguments of one scoring launch over n_tiles row tiles (256 rows each) for
-// all query tiles (128 queries each): the first n_tiles, or with `spread` that
-// many spaced evenly over the first `spread` tiles.
+// Arguments of one scoring launch over n_tiles row tiles (256 rows each), every
+// tile_step-th one from the first, for all query tiles (128 queries each).
 struct TcScoreArgs {
     uint32_t q_tiles = 0, k_chunks = 0;   // set by tc_score
     int terms = 1;                        // 1: plain BF16; 3: split (operands [hi | lo])
     uint32_t lo_col = 0;                  // set by tc_score: first column of the lo half
-    uint32_t n_tiles = 0, spread = 0;
+    uint32_t n_tiles = 0, tile_step = 1;
     uint32_t nq = 0, n = 0;               // valid queries / rows
     int metric = 0;
     const float* qnorm2 = nullptr;        // per query |q|^2 (L2)

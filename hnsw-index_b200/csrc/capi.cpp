@@ -1349,14 +1349,19 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     // candidates (about k n / rows per query, of a list of 32,768). n / 32 keeps
     // the sample's scoring and selection at a few percent of the candidate pass
     // (300 queries x 100k x 200 in BF16: 57 + 67 us with 16,384 rows). They are
-    // tiles spread over the base: rows are often stored cluster by cluster, and
-    // the first ones then say little about the others (500 queries x 400k x 96
-    // in 100 clusters stored in order, k = 10, BF16: 33,900 candidates per query
-    // and 2.55 ms a call from the first rows, 4,300 and 0.83 ms from spread
-    // tiles; 2,800 and 0.58 ms either way on shuffled rows).
+    // every tile_step-th tile of the base (at least 69 % of it is spanned): rows
+    // are often stored cluster by cluster, and the first ones then say little
+    // about the others (500 queries x 400k x 96 in 100 clusters stored in order,
+    // k = 10, BF16: 33,900 candidates per query and 2.55 ms a call from the first
+    // rows, 4,300 and 0.83 ms from spread tiles; 2,800 and 0.58 ms either way on
+    // shuffled rows). A step keeps the kernel's tile arithmetic to one product:
+    // spacing them by a division made the candidate pass 6.5 % slower.
     const uint32_t kk = std::min<uint32_t>(k, b->n);
-    const uint32_t sample_rows =
-        std::min<uint32_t>(np, std::min<uint32_t>(16384, round_up(std::max<uint32_t>({4096, b->n / 32, 64 * kk}), 256)));
+    const uint32_t tiles = np / 256;
+    const uint32_t most =
+        std::min<uint32_t>({tiles, 64u, round_up(std::max<uint32_t>({4096, b->n / 32, 64 * kk}), 256) / 256});
+    const uint32_t tile_step = std::max<uint32_t>(1, (tiles + most / 2) / most);
+    const uint32_t sample_rows = std::min<uint32_t>(most, (tiles + tile_step - 1) / tile_step) * 256;
     CU(b->dense.ensure(size_t(qp) * sample_rows * 4), "cudaMalloc sample");
     CU(b->thr1.ensure(size_t(qp) * 4), "cudaMalloc thresholds");
     CU(b->thr2.ensure(size_t(qp) * 4), "cudaMalloc thresholds");
@@ -1372,7 +1377,7 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     t.stall = b->stall;
     t.pairs = pairs ? 1u : 0u;
     t.n_tiles = sample_rows / 256;
-    t.spread = np / 256;
+    t.tile_step = tile_step;
     t.dense = b->dense.as<float>();
     t.ld = sample_rows;
     CU(tc_score(b->aop.as<__nv_bfloat16>(), qp, b->bop[ti].as<__nv_bfloat16>(), np, kp, t, b->num_sms, st), "sample pass");
@@ -1384,7 +1389,7 @@ static int brute_search_tensor(hnsw_gpu_brute* b, const float* queries, size_t n
     CU(b->cand.ensure(size_t(nq) * cap * 8), "cudaMalloc candidates");
     t.dense = nullptr;
     t.n_tiles = np / 256;
-    t.spread = 0;
+    t.tile_step = 1;
     t.thr = b->thr1.as<float>();
     t.cand_count = d_ccount;
     t.cand = b->cand.as<uint64_t>();
