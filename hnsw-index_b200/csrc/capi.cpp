@@ -180,7 +180,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
                           const uint32_t* d_fids,
                           uint64_t* d_keys, float* d_dist, uint32_t* d_count, int32_t* d_status, uint32_t ef_max,
                           uint32_t out_stride, cudaStream_t stream, const SearchGeometry* force, bool publish,
-                          bool reserve) {
+                          uint32_t load, bool reserve) {
     hnsw_search_opts o = o_in;
     if (o.mode != HNSW_MODE_PLAIN && o.mode != HNSW_MODE_PERSISTENT && o.mode != HNSW_MODE_AUTO)
         return set_error(HNSW_ERR_INVALID_ARGUMENT, "unknown search mode");
@@ -297,9 +297,11 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     // query) are decided on the device from their expected work, those whose
     // queries share one filter and one ef by the same rule here: their expected
     // work is equal, and ordering them would only cost the order kernel's time.
+    // The queries of a request loop's other batches (`load`) count as its own:
+    // they hold SMs that a team would have to itself otherwise.
     TeamGeometry team;
     const bool plans = o.exact_below > 0.0f && d_fbits, varied = d_efs || d_fbits;
-    const bool small = nq <= size_t(gi->num_sms) * (varied ? 2 : 4);
+    const bool small = nq + load <= size_t(gi->num_sms) * (varied ? 2 : 4);
     if (teams && !o.traversal && !plans && tags == 0 && (small || varied))
         CU(plan_search_team(a, ef_max, gi->num_sms, &team), "team occupancy");
     bool warp_route = !team.blocks || !small;
@@ -307,8 +309,8 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     if (team.blocks && !small && equal_work) {
         uint32_t warps = 0;
         CU(resident_search_warps(a, geo, gi->num_sms, &warps), "occupancy");
-        const float q = float(nq);
-        warp_route = kTeamSpeed * std::max(1.0f, q / float(warps)) <= std::max(1.0f, q / float(team.blocks));
+        const float q = float(nq + load);
+        warp_route = kTeamSpeed * std::max(1.0f, q / float(warps)) <= std::max(1.0f, q / float(team.resident));
         if (warp_route) team = TeamGeometry();
     }
     // Queries that outgrow a warp's scratch are redone by teams: a warp of the
@@ -386,8 +388,8 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         if (!a.persistent && warp_route) CU(resident_search_warps(a, geo, gi->num_sms, &slots), "occupancy");
         uint32_t* route = s->work.as<uint32_t>() + 5;
         if (!reserve)
-            CU(launch_query_order(a, s->order.as<uint32_t>(), s->order.as<uint8_t>() + nq * 4, slots, team.blocks,
-                                  route, stream),
+            CU(launch_query_order(a, s->order.as<uint32_t>(), s->order.as<uint8_t>() + nq * 4, slots,
+                                  team.resident, load, route, stream),
                "query order");
         a.order = s->order.as<uint32_t>();
         if (warp_route) a.route = route;
@@ -469,27 +471,29 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
     return HNSW_OK;
 }
 
-// Grows the slot's buffers to what batches of up to max_nq queries with a k
-// and an ef per query need, so that none of them allocates (growing a buffer
-// frees the old one, which waits for the batches of every other slot). The
-// schedule differs by ef bucket, and its smaller ones can need more memory
-// (more warps resident), so each is gone through: about 1 ms a slot.
+// Grows the slot's buffers to what a request loop's batches of up to max_nq
+// queries need, so that none of them allocates (growing a buffer frees the old
+// one, which waits for the batches of every other slot). The schedule differs
+// by ef bucket, and its smaller ones can need more memory (more warps
+// resident), so each is gone through: about 1 ms a slot.
 int hnswgpu::reserve_search(hnsw_gpu_index* gi, Slot* s, uint32_t max_nq, uint32_t max_ef, const hnsw_search_opts& o,
                             bool filtered) {
-    // Only whether these are given is looked at.
-    const uint32_t* given = reinterpret_cast<const uint32_t*>(s);
-    for (uint32_t nq : {max_nq, std::min<uint32_t>(max_nq, 2 * uint32_t(gi->num_sms))})
-        for (bool f : {false, true}) {
-            if (f && !filtered) continue;
+    // Batches alike, with a k and an ef per query, and with filters too; as
+    // large as can be, and as large as teams take whole, alone or beside others.
+    for (int kind = 0; kind < (filtered ? 3 : 2); ++kind) {
+        // Only whether these are given is looked at.
+        const uint32_t* given = kind > 0 ? reinterpret_cast<const uint32_t*>(s) : nullptr;
+        const uint64_t* bits = kind > 1 ? reinterpret_cast<const uint64_t*>(s) : nullptr;
+        const uint32_t whole = std::min<uint32_t>(max_nq, (kind > 0 ? 2 : 4) * uint32_t(gi->num_sms));
+        for (const auto& [nq, load] : {std::pair<uint32_t, uint32_t>{max_nq, 0}, {whole, 0}, {whole, max_nq}})
             for (uint32_t ef = std::min<uint32_t>(1056, max_ef);; ef -= 32) {
-                const uint32_t ef_max = ef > 1024 ? max_ef : ef;
-                int r = enqueue_search(gi, s, nullptr, nq, o, given, given,
-                                       f ? reinterpret_cast<const uint64_t*>(given) : nullptr, nullptr, nullptr, nullptr,
-                                       nullptr, nullptr, nullptr, ef_max, o.out_stride, s->stream, nullptr, true, true);
+                int r = enqueue_search(gi, s, nullptr, nq, o, given, given, bits, nullptr, nullptr, nullptr, nullptr,
+                                       nullptr, nullptr, ef > 1024 ? max_ef : ef, o.out_stride, s->stream, nullptr, true,
+                                       load, true);
                 if (r != HNSW_OK) return r;
                 if (ef <= 32) break;
             }
-        }
+    }
     return HNSW_OK;
 }
 

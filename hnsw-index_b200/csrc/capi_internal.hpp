@@ -358,13 +358,14 @@ struct hnsw_builder {
 
 namespace hnswgpu {
 // Enqueues one search on `stream` with device pointers. ef_max bounds every
-// per-query max(ef, k) of the batch. With `reserve` it only grows the slot's
-// buffers to what that search needs.
+// per-query max(ef, k) of the batch; `load` is the number of queries of other
+// batches that run beside it. With `reserve` it only grows the slot's buffers to
+// what that search needs.
 int enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_t nq, const hnsw_search_opts& o,
                    const uint32_t* d_ks, const uint32_t* d_efs, const uint64_t* d_fbits, const uint8_t* d_fused,
                    const uint32_t* d_fids, uint64_t* d_keys, float* d_dist, uint32_t* d_count, int32_t* d_status, uint32_t ef_max,
                    uint32_t out_stride, cudaStream_t stream, const SearchGeometry* force = nullptr,
-                   bool publish = false, bool reserve = false);
+                   bool publish = false, uint32_t load = 0, bool reserve = false);
 int reserve_search(hnsw_gpu_index* gi, Slot* s, uint32_t max_nq, uint32_t max_ef, const hnsw_search_opts& o,
                    bool filtered);
 // The ef bucket of the tuning table for a batch whose max(ef, k) is ef_max.

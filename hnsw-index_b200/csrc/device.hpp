@@ -196,19 +196,20 @@ struct TeamGeometry {
     uint32_t far_cap = 0;       // entries of a block's far list (args.team_far)
     uint32_t bitmap_words = 0;  // visited bitmap in shared memory; 0: in args.spill_bits, one row per block
     uint32_t blocks = 0;
+    uint32_t resident = 0;      // teams that the device holds at once (blocks: no more than queries)
     size_t smem = 0;
 };
 // Geometry for args.nq queries whose max(ef, k) is at most ef_max.
 cudaError_t plan_search_team(const SearchArgs& args, uint32_t ef_max, int num_sms, TeamGeometry* out);
 cudaError_t launch_search_team(const SearchArgs& args, const TeamGeometry& geo, cudaStream_t stream);
 // Query indices in descending order of expected work, and the kernel to take
-// the batch (kRoute*) given the warps or teams resident at once; `bucket` is
-// scratch (nq bytes).
+// the batch (kRoute*) given the warps or teams resident at once and `load` more
+// queries of its kind under way; `bucket` is scratch (nq bytes).
 constexpr uint32_t kRouteWarp = 1, kRouteTeam = 2;
 // A team's speed in warps (the comment at query_order_kernel has the figures).
 constexpr float kTeamSpeed = 2.2f;
 cudaError_t launch_query_order(const SearchArgs& args, uint32_t* order, uint8_t* bucket, uint32_t warp_slots,
-                               uint32_t team_slots, uint32_t* route, cudaStream_t stream);
+                               uint32_t team_slots, uint32_t load, uint32_t* route, cudaStream_t stream);
 
 constexpr uint32_t kColdChunkShift = 10;
 constexpr uint32_t kColdChunk = 1u << kColdChunkShift;  // entries per cold chunk (8 KB)

@@ -992,14 +992,16 @@ __device__ __forceinline__ float expected_work(const SearchArgs& a, uint32_t qi)
 // route of the batch: a warp or a team per query. One block.
 //
 // The route compares the two kernels' expected times: the longest query's or
-// the whole work over the resident warps or teams, whichever is more. A team
+// the whole work over the resident warps or teams, whichever is more (a request
+// loop's other batches add `load` queries of the batch's mean work). A team
 // takes about 2.2 times fewer cycles per expansion than a warp (3,000 filtered
 // int8 queries on 100k x 96 with 1-90 % selectivity: 2.1k against 4.6k), so it
 // wins where the longest query decides (that batch: 55 against 143 ms) and
 // loses where the SMs are full of queries of like length (592 teams or 2,368
 // warps: 4,000 unfiltered queries at ef = 64 take 1.47 against 1.00 ms).
 __global__ void __launch_bounds__(1024) query_order_kernel(SearchArgs a, uint32_t* order, uint8_t* bucket,
-                                                           float warp_slots, float team_slots, uint32_t* route) {
+                                                           float warp_slots, float team_slots, float load,
+                                                           uint32_t* route) {
     constexpr uint32_t B = 128;
     __shared__ uint32_t hist[B], next[B];
     __shared__ float wsum[32], wmax[32];
@@ -1034,6 +1036,7 @@ __global__ void __launch_bounds__(1024) query_order_kernel(SearchArgs a, uint32_
             sum += wsum[i];
             mx = fmaxf(mx, wmax[i]);
         }
+        sum += sum * load / float(a.nq);
         *route = kTeamSpeed * fmaxf(mx, sum / warp_slots) > fmaxf(mx, sum / team_slots) ? kRouteTeam : kRouteWarp;
     }
     __syncthreads();
@@ -1081,7 +1084,8 @@ cudaError_t plan_search_team(const SearchArgs& a, uint32_t ef_max, int num_sms, 
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, int(32 * g.warps), g.smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaSuccess;
-    g.blocks = std::min<uint32_t>(a.nq, uint32_t(num_sms) * uint32_t(per_sm));
+    g.resident = uint32_t(num_sms) * uint32_t(per_sm);
+    g.blocks = std::min<uint32_t>(a.nq, g.resident);
     // Far lists: one entry per node at most, 256 MB in all (a query that
     // needs more goes to the retry pass).
     g.far_cap = std::min<uint32_t>((a.ix.n + 31) / 32 * 32, std::min<uint32_t>(1u << 18, (1u << 25) / g.blocks));
@@ -1095,8 +1099,9 @@ cudaError_t launch_search_team(const SearchArgs& a, const TeamGeometry& g, cudaS
 }
 
 cudaError_t launch_query_order(const SearchArgs& a, uint32_t* order, uint8_t* bucket, uint32_t warp_slots,
-                               uint32_t team_slots, uint32_t* route, cudaStream_t stream) {
-    dev::query_order_kernel<<<1, 1024, 0, stream>>>(a, order, bucket, float(warp_slots), float(team_slots), route);
+                               uint32_t team_slots, uint32_t load, uint32_t* route, cudaStream_t stream) {
+    dev::query_order_kernel<<<1, 1024, 0, stream>>>(a, order, bucket, float(warp_slots), float(team_slots),
+                                                    float(load), route);
     return cudaGetLastError();
 }
 

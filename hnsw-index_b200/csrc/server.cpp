@@ -135,11 +135,12 @@ void reserve_slot(hnsw_gpu_server* s, Slot* sl, size_t* budget) {
     *budget -= std::min(*budget, before > after ? before - after : 0);
 }
 
-int stage_and_launch(hnsw_gpu_server* s, BatchSlot& b, std::vector<uint64_t>& tickets) {
+// `load`: queries of the batches in flight that have not finished.
+int stage_and_launch(hnsw_gpu_server* s, BatchSlot& b, std::vector<uint64_t>& tickets, uint32_t load) {
     TraceRange trace("hnsw.server_batch");
     const uint32_t n = uint32_t(tickets.size());
     const uint32_t dim = s->dim, K = s->cfg.max_k;
-    bool any_filter = false;
+    bool any_filter = false, alike = true;
     uint32_t ef_max = 1;
     for (uint32_t i = 0; i < n; ++i) {
         Request& r = s->at(tickets[i]);
@@ -151,15 +152,19 @@ int stage_and_launch(hnsw_gpu_server* s, BatchSlot& b, std::vector<uint64_t>& ti
         b.h_fused[i] = r.filter_id >= 0 ? 1 : 0;
         b.h_fids[i] = r.filter_id >= 0 ? uint32_t(r.filter_id) : 0u;
         any_filter |= r.filter_id >= 0;
+        alike = alike && r.k == b.h_ks[0] && r.ef == b.h_efs[0];
     }
+    alike = alike && !any_filter;
     Slot* sl = b.slot;
     cudaStream_t st = sl->stream;
     CU(sl->q.ensure(size_t(s->cfg.max_batch) * dim * 4), "server queries");
     CU(sl->ks.ensure(size_t(s->cfg.max_batch) * 4), "server ks");
     CU(sl->efs.ensure(size_t(s->cfg.max_batch) * 4), "server efs");
     CU(cudaMemcpyAsync(sl->q.p, b.h_q, size_t(n) * dim * 4, cudaMemcpyHostToDevice, st), "copy queries");
-    CU(cudaMemcpyAsync(sl->ks.p, b.h_ks, size_t(n) * 4, cudaMemcpyHostToDevice, st), "copy ks");
-    CU(cudaMemcpyAsync(sl->efs.p, b.h_efs, size_t(n) * 4, cudaMemcpyHostToDevice, st), "copy efs");
+    if (!alike) {
+        CU(cudaMemcpyAsync(sl->ks.p, b.h_ks, size_t(n) * 4, cudaMemcpyHostToDevice, st), "copy ks");
+        CU(cudaMemcpyAsync(sl->efs.p, b.h_efs, size_t(n) * 4, cudaMemcpyHostToDevice, st), "copy efs");
+    }
     const uint64_t* d_fb = nullptr;
     const uint8_t* d_fu = nullptr;
     const uint32_t* d_fi = nullptr;
@@ -172,12 +177,17 @@ int stage_and_launch(hnsw_gpu_server* s, BatchSlot& b, std::vector<uint64_t>& ti
         d_fu = sl->fused.as<uint8_t>();
         d_fi = sl->fids.as<uint32_t>();
     }
-    const hnsw_search_opts o = server_opts(s);
+    hnsw_search_opts o = server_opts(s);
+    if (alike) {  // one k and one ef for the batch: no route or order to work out
+        o.k = b.h_ks[0];
+        o.ef = b.h_efs[0];
+    }
     b.finished.assign(n, 0);
     b.remaining = n;
     // Scratch sized for the batch's own largest max(ef, k).
-    int r = enqueue_search(s->index, sl, sl->q.as<float>(), n, o, sl->ks.as<uint32_t>(), sl->efs.as<uint32_t>(), d_fb,
-                           d_fu, d_fi, b.d_keys, b.d_dist, b.d_count, b.d_status, ef_max, K, st, nullptr, true);
+    int r = enqueue_search(s->index, sl, sl->q.as<float>(), n, o, alike ? nullptr : sl->ks.as<uint32_t>(),
+                           alike ? nullptr : sl->efs.as<uint32_t>(), d_fb, d_fu, d_fi, b.d_keys, b.d_dist, b.d_count,
+                           b.d_status, ef_max, K, st, nullptr, true, load);
     if (r != HNSW_OK) return r;
     CU(cudaEventRecord(b.done, st), "record batch event");
     return HNSW_OK;
@@ -260,9 +270,11 @@ void dispatch_loop(hnsw_gpu_server* s) {
                 s->at(t).state = ReqState::Inflight;
                 take.push_back(t);
             }
+            uint32_t load = 0;
+            for (const BatchSlot& b : s->batches) load += b.busy ? b.remaining : 0;
             free_slot->busy = true;
             free_slot->tickets = take;
-            const int r = stage_and_launch(s, *free_slot, free_slot->tickets);
+            const int r = stage_and_launch(s, *free_slot, free_slot->tickets, load);
             ++s->launched_batches;
             s->launched_queries += take.size();
             if (r != HNSW_OK) {

@@ -245,7 +245,7 @@ int hnsw_gpu_read_counters(hnsw_gpu_index* index, uint32_t* host_out, size_t nq)
  * as soon as one of max_inflight device scratch slots is free, so requests
  * arriving while earlier batches run join the next launch and overlap on the
  * device. Each result equals the same search run alone. The start allocates
- * every slot's device scratch for max_batch, max_k and max_ef (6.3 GB a slot
+ * every slot's device scratch for max_batch, max_k and max_ef (6.6 GB a slot
  * at 10M x 128 with filters, most of it one bit per node for each resident
  * warp), at most half of the free memory in all; slots past that grow as they
  * go, and the index keeps the scratch after the stop. */

@@ -185,3 +185,28 @@ def test_batches_of_rising_size_allocate_nothing(served):
         srv.stop()
         gi.close()
     assert free[2] - free[3] <= 4 << 20
+
+
+@pytest.mark.parametrize("gap_us", [0.0, 0.4, 20.0])
+def test_alike_and_mixed_batches_beside_others(served, gap_us):
+    """Requests with one k and ef (whose batches carry neither per query) before
+    and after mixed ones, alone on the device or with several batches in
+    flight, which moves small batches from teams to the warp kernels."""
+    base, queries, data = served
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    n = 2400
+    q = np.tile(queries, (4, 1))
+    ks, efs, fids, bank = make_requests(q, 20000, 9)
+    alike = (np.arange(n) // 600) % 2 == 0
+    ks[alike], efs[alike], fids[alike] = 10, 64, -1
+    srv = H.Server(gi, max_batch=200, max_inflight=6, max_pending=1 << 14, max_k=100, max_ef=512, linger_us=20,
+                   filter_nbits=20000, filter_bank=bank)
+    keys, dist, cnt, st, _ = srv.replay(q, np.arange(n) * gap_us, ks, efs, fids)
+    srv.stop()
+    rk, rd, rc, rs = oracle_results(oi, q, ks, efs, fids, bank, 20000)
+    np.testing.assert_array_equal(st, rs)
+    np.testing.assert_array_equal(cnt, rc)
+    for i in range(n):
+        c = int(rc[i])
+        np.testing.assert_array_equal(keys[i, :c], rk[i, :c])
+        np.testing.assert_array_equal(dist[i, :c].view(np.uint32), rd[i, :c].view(np.uint32))
