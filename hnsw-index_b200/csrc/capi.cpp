@@ -430,6 +430,7 @@ int hnswgpu::enqueue_search(hnsw_gpu_index* gi, Slot* s, const float* d_q, size_
         CU(cudaMemcpy(s->last_tab.p, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice), "copy last-resort table");
     }
     if (reserve) return HNSW_OK;
+    s->taken_by = !team.blocks ? Slot::kWarps : (warp_route ? Slot::kDevice : Slot::kTeams);
     a.overflow_list2 = s->overflow2.as<uint32_t>();
     a.overflow_count2 = s->work.as<uint32_t>() + 4;
     if (plans) {
@@ -977,6 +978,7 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
     // heuristic's is timed as a search on an untuned index runs (teams where
     // the batch takes them), the others on the warp kernels alone.
     const SearchGeometry automatic{0, 0, 0, 0, 0};
+    bool by_teams[2] = {false, false};  // whether teams took the heuristic's trial
     auto timed = [&](const SearchGeometry& g, int32_t mode, int32_t heuristic, float* ms) {
         hnsw_search_opts ot = o;
         ot.mode = mode;
@@ -1006,6 +1008,17 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
         std::sort(sorted.begin(), sorted.end());
         *ms = sorted[reps / 2];
         trials.push_back({g, mode, heuristic, *ms});
+        if (heuristic && s->taken_by != Slot::kWarps) {
+            uint32_t route = kRouteTeam;
+            if (s->taken_by == Slot::kDevice) {
+                const cudaError_t e = cudaMemcpy(&route, s->work.as<uint32_t>() + 5, 4, cudaMemcpyDeviceToHost);
+                if (e != cudaSuccess) {
+                    r = cuda_fail(e, "autotune route");
+                    return false;
+                }
+            }
+            by_teams[mode] = route == kRouteTeam;
+        }
         return true;
     };
     for (int32_t mode : {HNSW_MODE_PLAIN, HNSW_MODE_PERSISTENT}) {
@@ -1065,8 +1078,15 @@ int hnsw_gpu_autotune(hnsw_gpu_index* gi, const float* queries, size_t nq, size_
     {
         std::lock_guard<std::mutex> l(gi->tune_mu);
         hnsw_gpu_index::Tuned& slot = gi->tuned[tune_bucket(ef_bound)];
-        for (int m : {0, 1}) slot.geo[m] = win[m]->heuristic ? automatic : win[m]->g;
-        slot.mode = top->mode;
+        slot = hnsw_gpu_index::Tuned();
+        // A sample that teams take in both modes says nothing about the warp
+        // kernels of either, and picking a mode from it would be picking one by
+        // noise (5M x 96, 8,000 queries: 206.5 ms in both; 50,000, of which the
+        // warp kernels take part: 1.36 s plain, 0.81 persistent).
+        if (!by_teams[0] || !by_teams[1]) {
+            for (int m : {0, 1}) slot.geo[m] = win[m]->heuristic ? automatic : win[m]->g;
+            slot.mode = top->mode;
+        }
     }
     auto fill = [](const Trial& t, hnsw_tune_entry* e) {
         e->schedule.ef_cap = t.g.ef_cap;

@@ -187,6 +187,9 @@ struct Slot {
     DBuf planned;                         // selectivity planner flags
     DBuf team_bits, team_far, order;      // team traversal: visited bitmaps, far candidates, query order
     size_t last_nq = 0;
+    // Who took the last search: the warp kernel, teams, or whom the device's
+    // route word (work[5]) names.
+    enum { kWarps, kTeams, kDevice } taken_by = kWarps;
     ~Slot() {
         for (DBuf* b : {&q, &ks, &efs, &fbits, &fused, &fids, &work, &overflow, &counters,
                         &g_results, &g_cands, &g_visited, &spill_bits, &spill_cands, &cold_pool, &cold_tab, &last_pool,

@@ -207,16 +207,17 @@ int hnsw_gpu_set_schedule(hnsw_gpu_index* index, const hnsw_schedule* schedule);
  * hnsw_gpu_search_batch) under every feasible schedule of the grid
  * mode x warps per block {1, 2, 4, 8} x visited-hash size {16, 32, 64} x
  * ef_cap (rounded up to a multiple of 64, 1024..32768 entries) x staged
- * rows, by coordinate descent from the heuristic's own choice, `reps` timed runs each after one warm-up (median,
- * CUDA events). The heuristic's entry is timed as an untuned search runs (with
- * a team of warps per query where the batch takes them), the others on the
- * one-warp kernels. Unless the heuristic won, the fastest schedule of each
- * mode is stored in the index's tuning table for the ef bucket of the sample's
- * max(ef, k) (buckets of 32), used from then on by the one-warp kernels of
- * searches in that bucket unless a fixed schedule is set (which also keeps
- * every search on those kernels); HNSW_MODE_AUTO picks the faster mode.
- * Results never depend on the schedule. `entries` (optional, `cap` entries)
- * receives every trial. */
+ * rows, by coordinate descent from the heuristic's own choice, `reps` timed
+ * runs each after one warm-up (median, CUDA events). The heuristic's entry is
+ * timed as an untuned search runs (with a team of warps per query where the
+ * batch takes them), the others on the one-warp kernels. Unless the heuristic
+ * won, or teams took the sample in both modes (nothing is stored then), the
+ * fastest schedule of each mode is stored in the index's tuning table for the
+ * ef bucket of the sample's max(ef, k) (buckets of 32), used from then on by
+ * the one-warp kernels of searches in that bucket unless a fixed schedule is
+ * set (which also keeps every search on those kernels); HNSW_MODE_AUTO picks
+ * the faster mode. Results never depend on the schedule. `entries` (optional,
+ * `cap` entries) receives every trial. */
 typedef struct hnsw_tune_entry {
     hnsw_schedule schedule;
     int32_t mode;  /* HNSW_MODE_PLAIN or HNSW_MODE_PERSISTENT */
