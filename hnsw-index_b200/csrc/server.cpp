@@ -8,8 +8,8 @@
 // while earlier batches run are admitted and their work overlaps on the
 // device. When every slot is busy, requests wait on the host; when the
 // pending queue is full, submission is rejected (ADMISSION_REJECTED). A batch
-// runs the persistent search kernel with per-query k, ef and filters, so each
-// result equals the result of the same search run alone. The kernel writes
+// is searched with per-query k, ef and filters, by the persistent kernel or by
+// teams of warps, so each result equals that of the same search run alone. The kernels write
 // each query's results into mapped host memory and publishes its status last,
 // so a request completes when its own query does, not when its batch does.
 #include <algorithm>
