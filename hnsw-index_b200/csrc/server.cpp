@@ -9,9 +9,10 @@
 // device. When every slot is busy, requests wait on the host; when the
 // pending queue is full, submission is rejected (ADMISSION_REJECTED). A batch
 // is searched with per-query k, ef and filters, by the persistent kernel or by
-// teams of warps, so each result equals that of the same search run alone. The kernels write
-// each query's results into mapped host memory and publishes its status last,
-// so a request completes when its own query does, not when its batch does.
+// teams of warps, so each result equals that of the same search run alone. The
+// kernels write each query's results into mapped host memory and publish its
+// status last, so a request completes when its own query does, not when its
+// batch does.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
