@@ -81,10 +81,12 @@ struct DBuf {
 // through pinned memory (a copy to pageable memory costs about 10 us however
 // small it is: 1 query's four arrays took 40 of 183 us); larger ones, where
 // the bytes decide, go to the caller's arrays directly. So does the first
-// call's result: the pinned buffer costs 1.3 ms, which only a handle that is
-// used again gets back.
+// call's result: the driver pins 2 MB at a time, which costs 1.3 to 3 ms that only a
+// handle that is used again gets back, unless another handle's buffer holds
+// such a chunk already (a small buffer then takes about 5 us).
+inline std::atomic<int> g_pinned_outputs{0};  // handles' pinned buffers alive
 struct Outputs {
-    static constexpr size_t kStaged = size_t(1) << 20;
+    static constexpr size_t kStaged = size_t(1) << 20, kSmall = size_t(1) << 18;
     DBuf dev;
     void* host = nullptr;
     size_t host_bytes = 0, rows = 0, stride = 0, tail = 0;
@@ -125,17 +127,21 @@ struct Outputs {
     cudaError_t fetch(cudaStream_t st, uint64_t* k, float* d, uint32_t* c, int32_t* s, bool rows_out = true,
                       void* extra_out = nullptr) {
         const size_t kb = rows_out ? rows * stride * 8 : 0, db = rows_out ? rows * stride * 4 : 0;
-        const bool first = !used;
+        const bool staged =
+            bytes() <= kStaged && (used || (bytes() <= kSmall && g_pinned_outputs.load(std::memory_order_relaxed) > 0));
         used = true;
-        if (bytes() <= kStaged && !first) {
+        if (staged) {
             if (host_bytes < bytes()) {
-                if (host) cudaFreeHost(host);
-                host = nullptr;
-                host_bytes = 0;
+                release_host();
                 size_t want = 16384;
                 while (want < bytes()) want <<= 1;
-                if (cudaHostAlloc(&host, want, cudaHostAllocDefault) == cudaSuccess) host_bytes = want;
-                else cudaGetLastError();  // no pinned memory: copy directly
+                if (cudaHostAlloc(&host, want, cudaHostAllocDefault) == cudaSuccess) {
+                    host_bytes = want;
+                    g_pinned_outputs.fetch_add(1, std::memory_order_relaxed);
+                } else {
+                    host = nullptr;
+                    cudaGetLastError();  // no pinned memory: copy directly
+                }
             }
             if (host_bytes >= bytes()) {
                 cudaError_t e = cudaMemcpyAsync(host, dev.p, bytes(), cudaMemcpyDeviceToHost, st);
@@ -165,11 +171,16 @@ struct Outputs {
         if (e == cudaSuccess && rows_out && !cleared) zero_unfilled(k, d, c, s);
         return e;
     }
-    void release() {
-        dev.release();
-        if (host) cudaFreeHost(host);
+    void release_host() {
+        if (!host) return;
+        cudaFreeHost(host);
+        g_pinned_outputs.fetch_sub(1, std::memory_order_relaxed);
         host = nullptr;
         host_bytes = 0;
+    }
+    void release() {
+        dev.release();
+        release_host();
     }
 };
 
