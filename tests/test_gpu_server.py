@@ -210,3 +210,23 @@ def test_alike_and_mixed_batches_beside_others(served, gap_us):
         c = int(rc[i])
         np.testing.assert_array_equal(keys[i, :c], rk[i, :c])
         np.testing.assert_array_equal(dist[i, :c].view(np.uint32), rd[i, :c].view(np.uint32))
+
+
+def test_server_without_memory_for_its_slots_serves_all_the_same(served):
+    """The slots are reserved when the server starts; without memory for that
+    they grow with the batches, as in any other call."""
+    base, queries, data = served
+    gi, oi = H.HnswIndex.from_bytes(data), O.Index(data)
+    try:
+        H.debug_fail_allocations(1)
+        srv = H.Server(gi, max_batch=256, max_inflight=3, max_pending=4096, max_k=10, max_ef=128, linger_us=50)
+    finally:
+        H.debug_fail_allocations(0)
+    n = len(queries)
+    ks, efs = np.full(n, 10, np.uint32), (np.arange(n) % 97 + 16).astype(np.uint32)
+    keys, _, cnt, st, _ = srv.replay(queries, np.zeros(n), ks, efs)
+    srv.stop()
+    rk, _, rc, rs = oi.search(queries, 10, 16, ks=ks, efs=efs)
+    np.testing.assert_array_equal(st, rs)
+    np.testing.assert_array_equal(cnt, rc)
+    np.testing.assert_array_equal(keys[:, :10], rk)
